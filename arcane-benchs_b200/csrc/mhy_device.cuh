@@ -9,6 +9,7 @@
 
 #include <cstdint>
 #include "mhy_pow_third.h"
+#include "mhy_quot.h"
 
 namespace mhy {
 
@@ -57,37 +58,28 @@ __device__ __forceinline__ double qdiv(double x, double y, double r) {
   return __fma_rn(__fma_rn(-q0, y, x), r, q0);
 }
 
-// The sweeps' speculative form of qdiv: the corrected quotient (or q0 for a
-// zero numerator) without a branch, and a flag when it may differ from
-// x / y: a zero x over a y that is not a normal number; otherwise x or q0
-// outside 2^-960 <= |.| < 2^960 (zeros, subnormals, huge values, inf, NaN)
-// or y outside 2^-959 <= |y| < 2^960, all tested on the biased exponents.
-// A warp whose lanes raised the flag recomputes its segment with qdiv (the
-// sweeps' *_line_exact functions), so the results are x / y bit for bit
-// either way.  Measured on Sedov 128^3 FP64: no warp raised the flag in 505
-// cycles, and the cycle takes 1.21 ms instead of 1.32 ms with qdiv's
-// branches.  (Scaling tiny numerators by 2^200 first, so that a field's
-// subnormal tail would stay on the fast path, cost 3 % more and was left out.)
-__device__ __forceinline__ double qdiv_spec(double x, double y, double r, unsigned& oor) {
-  const double q0 = x * r;
-  const double q = __fma_rn(__fma_rn(-q0, y, x), r, q0);
-  const unsigned bx = (unsigned)__double2hiint(x) >> 20 & 0x7ffu;
-  const unsigned by = (unsigned)__double2hiint(y) >> 20 & 0x7ffu;
-  const unsigned bq0 = (unsigned)__double2hiint(q0) >> 20 & 0x7ffu;
-  const bool zero = x == 0.0;
-  const bool bad = zero ? by - 1u > 2045u : (bx - 63u > 1919u || by - 64u > 1918u || bq0 - 63u > 1919u);
-  oor |= bad ? 1u : 0u;
-  return zero ? q0 : q;
+// The sweeps' quotients.  FP32 (the mixed form) takes the product with the
+// reciprocal; FP64 takes qdiv, or in its speculative form (SP) the branch-free
+// quotient of mhy_quot.h, which raises *oor where it may differ from x / y.  A
+// thread (or warp) that raised it does its work again with SP off, so the
+// results are x / y bit for bit either way.
+template <typename R, bool SP>
+__device__ __forceinline__ R rc(R y, unsigned* oor) {
+  if constexpr (sizeof(R) == 8 && SP) return rcp_fast(y, *oor);
+  else return R(1) / y;
 }
-
-// Quotient x / y with r = 1 / y at hand in the sweeps: FP32 (the mixed form)
-// takes the product; FP64 takes qdiv, or its speculative form (SP) with the
-// flag in *oor.
 template <typename R, bool SP>
 __device__ __forceinline__ R dv(R x, R y, R r, unsigned* oor) {
   if constexpr (sizeof(R) == 4) return x * r;
-  else if constexpr (SP) return qdiv_spec(x, y, r, *oor);
+  else if constexpr (SP) return quo_from_rcp(x, y, r, *oor);
   else return qdiv(x, y, r);
+}
+// A quotient with a denominator of its own.
+template <typename R, bool SP>
+__device__ __forceinline__ R qu(R x, R y, unsigned* oor) {
+  if constexpr (sizeof(R) == 4) return __fdividef(x, y);
+  else if constexpr (SP) return quo_fast(x, y, *oor);
+  else return x / y;
 }
 
 // Arcane math::min / math::max and std::min / std::max, as the reference writes them
@@ -136,37 +128,73 @@ __device__ __forceinline__ R flux_limiter_g(int id, R gradplus, R gradmoins, R y
   return grady;
 }
 
-template <typename R>
-__device__ __forceinline__ R limiter(int id, R r) {
+template <typename R, bool SP = false>
+__device__ __forceinline__ R limiter(int id, R r, unsigned* oor = nullptr) {
   switch (id) {
     case 0: return tmax(R(0), tmin(R(1), r));
     case 1: return tmax(R(0), tmax(tmin(R(2) * r, R(1)), tmin(r, R(2))));
-    case 2: return (r <= R(0) ? R(0) : R(2) * r / (R(1) + r));
+    case 2:
+      if constexpr (sizeof(R) == 8 && SP) return r <= R(0) ? R(0) : qu<R, SP>(R(2) * r, R(1) + r, oor);
+      else return (r <= R(0) ? R(0) : R(2) * r / (R(1) + r));
     default: return R(0);
   }
 }
 
-// Arithmetic of the remap evaluation in precision R.  double: the reference's
-// operations exactly (qdiv gives x / y bit for bit).  float (the mixed
-// precision form): one reciprocal per shared denominator and products.
-template <typename R> struct Ar;
-template <> struct Ar<double> {
-  __device__ static __forceinline__ double rcp(double y) { return 1.0 / y; }
-  __device__ static __forceinline__ double div(double x, double y, double r) { return qdiv(x, y, r); }
-  __device__ static __forceinline__ double quo(double x, double y) { return x / y; }
-};
-template <> struct Ar<float> {
-  __device__ static __forceinline__ float rcp(float y) { return 1.0f / y; }
-  __device__ static __forceinline__ float div(float x, float, float r) { return x * r; }
-  __device__ static __forceinline__ float quo(float x, float y) { return __fdividef(x, y); }
-};
+// The limited slope of the remap from the back and front differences gb, gf
+// (RemapADIService.cc:497-506 and DualPhaseRemap.cc:736-777):
+//   g = 0; if (gb != 0) g += 0.5 phi(gf/gb) gb; if (gf != 0) g += 0.5 phi(gb/gf) gf.
+// DUAL: the products associate as (0.5 phi) g, else as 0.5 (phi g).
+// For minmod, phi(r) = max(0, min(1, r)): with finite gb, gf of opposite signs or
+// a zero the two terms are signed zeros and g = +0; with equal signs the ratio
+// whose numerator is the smaller magnitude is the only one below 1, the other
+// term is exactly 0.5 g.  So one division gives the reference's bits.  For
+// superBee and vanLeer the speculative form takes the same g = +0 for
+// differences of opposite signs or a zero, and raises *oor for differences of
+// 1e150 and more, infinities and NaN, whose terms may be other than zero.
+template <typename R, bool DUAL, bool SP>
+__device__ __forceinline__ R limited_slope(int lim, R gb, R gf, unsigned* oor) {
+  const R h = R(0.5), one = R(1), zero = R(0);
+  if (lim == 0) {
+    if constexpr (sizeof(R) == 8 && SP) {
+      const bool live = !(gb == zero || gf == zero || ((gb > zero) != (gf > zero)));
+      const bool fsmall = fabs(gf) < fabs(gb);
+      const R num = fsmall ? gf : gb, den = fsmall ? gb : gf;
+      unsigned bad = 0u;
+      const R r = quo_fast(num, den, bad);
+      if (live) *oor |= bad;
+      const R t1 = DUAL ? h * r * den : h * (r * den), t2 = DUAL ? h * one * num : h * (one * num);
+      return live ? (zero + t1) + t2 : zero;
+    } else {
+      if (gb == zero || gf == zero || ((gb > zero) != (gf > zero))) return zero;
+      const bool fsmall = fabs(gf) < fabs(gb);
+      const R r = fsmall ? qu<R, false>(gf, gb, nullptr) : qu<R, false>(gb, gf, nullptr);
+      const R t1 = fsmall ? (DUAL ? h * r * gb : h * (r * gb)) : (DUAL ? h * one * gb : h * (one * gb));
+      const R t2 = fsmall ? (DUAL ? h * one * gf : h * (one * gf)) : (DUAL ? h * r * gf : h * (r * gf));
+      return (zero + t1) + t2;
+    }
+  }
+  if constexpr (sizeof(R) == 8 && SP) {
+    if (!(fabs(gb) < 1e150 && fabs(gf) < 1e150)) *oor = 1u;
+    if (lim < 0 || (gb <= zero && gf >= zero) || (gb >= zero && gf <= zero)) return zero;   // lim < 0: order 1
+    const R rb = quo_fast(gf, gb, *oor), rf = quo_fast(gb, gf, *oor);
+    const R pb = limiter<R, true>(lim, rb, oor), pf = limiter<R, true>(lim, rf, oor);
+    return (zero + (DUAL ? h * pb * gb : h * (pb * gb))) + (DUAL ? h * pf * gf : h * (pf * gf));
+  } else {
+    R g = zero;
+    if (gb != zero) { const R p = limiter<R>(lim, qu<R, false>(gf, gb, nullptr)); g += DUAL ? h * p * gb : h * (p * gb); }
+    if (gf != zero) { const R p = limiter<R>(lim, qu<R, false>(gb, gf, nullptr)); g += DUAL ? h * p * gf : h * (p * gf); }
+    return g;
+  }
+}
 
 // Equations of state.  After the remap, p and c from rho and e:
 // PerfectGas (eos/perfectgas/PerfectGasEOSService.cc:92-106) and StiffenedGas
 // (eos/stiffenedgas/StiffenedGasEOSService.cc:29-44, pinf = limit-tension).
-__device__ __forceinline__ void eos_pc(int kind, double g, double pinf, double r, double e, double& p, double& c) {
-  if (kind == 1) { p = ((g - 1.) * r * e) - (g * pinf); c = sqrt((g / r) * (p + pinf)); }
-  else { p = (g - 1.) * r * e; c = sqrt(g * p / r); }
+template <bool SP = false>
+__device__ __forceinline__ void eos_pc(int kind, double g, double pinf, double r, double e, double& p, double& c,
+                                       unsigned* oor = nullptr) {
+  if (kind == 1) { p = ((g - 1.) * r * e) - (g * pinf); c = sqrt(qu<double, SP>(g, r, oor) * (p + pinf)); }
+  else { p = (g - 1.) * r * e; c = sqrt(qu<double, SP>(g * p, r, oor)); }
 }
 // initEOS: e and c from rho and p (PerfectGasEOSService.cc:20-32,
 // StiffenedGasEOSService.cc:10-24).

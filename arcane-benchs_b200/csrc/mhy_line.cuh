@@ -67,16 +67,16 @@ __device__ __forceinline__ void finalize_cell(const Phys& ph, const Scalars* S, 
   const double thr = ph.threshold;
   const double U0 = u[0], U1 = u[1], U2 = u[2], U3 = u[3];
   const double volt = 0. + U0, masset = 0. + U1;
-  const double unsurvolt = 1. / volt;
-  const double unsurvol = 1. / vol;
+  const double unsurvolt = rc<double, SP>(volt, oor);
+  const double unsurvol = rc<double, SP>(vol, oor);
   double fvol = U0 * unsurvolt;
   if (fvol < thr) fvol = 0.;
   const double somme_frac = 0. + fvol;
   const double unsursomme_frac = 1. / somme_frac;
   fvol = fvol * unsursomme_frac;
-  double mf = 1.;
+  double mf = 1., unsurmasset = 0.;
   if (masset != 0.) {
-    const double unsurmasset = 1. / masset;
+    unsurmasset = rc<double, SP>(masset, oor);
     mf = U1 * unsurmasset;
     if (fvol < thr) mf = 0.;
     const double fmasset = 0. + mf;
@@ -85,11 +85,11 @@ __device__ __forceinline__ void finalize_cell(const Phys& ph, const Scalars* S, 
     atomicOr(&const_cast<Scalars*>(S)->status, MHY_STATUS_ZERO_MASS);
   }
   double de = 0.;
-  if (fvol > thr) { const double vn = U0 * vol * unsurvolt; de = U1 / vn; }
+  if (fvol > thr) { const double vn = U0 * vol * unsurvolt; de = qu<double, SP>(U1, vn, oor); }
   const double density_nplus1 = 0. + fvol * de;
   const double cm = vol * density_nplus1;
   double ee = 0.;
-  if (fvol > thr && U1 != 0.) ee = dv<double, SP>(U2, U1, 1. / masset, oor);   // masset = 0 + U1 = U1
+  if (fvol > thr && U1 != 0.) ee = dv<double, SP>(U2, U1, unsurmasset, oor);   // masset = 0 + U1 = U1
   double energie = 0. + mf * ee;
   const double pv = U3 * unsurvol;
   const double pseudo = 0. + fvol * pv;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void finalize_cell(const Phys& ph, const Scalars* S, 
   out[7] = mf;
   if (r < 0. || energie < 0.) { energie = 0.; r = 0.; out[7] = 0.; }   // RemapADIFinal.cc:611-626
   double pr, cc;
-  eos_pc(ph.eos, ph.gamma, ph.pinf, r, energie, pr, cc);
+  eos_pc<SP>(ph.eos, ph.gamma, ph.pinf, r, energie, pr, cc, oor);
   out[0] = r;
   out[1] = energie;
   out[2] = pseudo;
@@ -141,7 +141,7 @@ __device__ __forceinline__ void finalize_cell_mixed(const Phys& ph, const Scalar
 // (RemapADIService.cc:962-970, PrepareRemap.cc:394-398); Phi0 = U0/U0 = 1.
 template <typename R, bool SP = false>
 __device__ __forceinline__ void phi_of(const double U[4], R P[4], unsigned* oor = nullptr) {
-  const R U0 = (R)U[0], r = Ar<R>::rcp(U0);
+  const R U0 = (R)U[0], r = rc<R, SP>(U0, oor);
   P[0] = 1;
   P[1] = dv<R, SP>((R)U[1], U0, r, oor); P[2] = dv<R, SP>((R)U[2], U0, r, oor); P[3] = dv<R, SP>((R)U[3], U0, r, oor);
 }
@@ -150,45 +150,28 @@ __device__ __forceinline__ void phi_of(const double U[4], R P[4], unsigned* oor 
 template <typename R, bool SP = false>
 __device__ __forceinline__ void face_grad(bool inner, R dx, const R Pn[4], const R Pp[4], R g[4], unsigned* oor = nullptr) {
   g[0] = 0;
-  const R r = inner ? Ar<R>::rcp(dx) : R(0);
   unsigned fo = 0u;
+  const R r = inner ? rc<R, SP>(dx, &fo) : R(0);
 #pragma unroll
   for (int v = 1; v < 4; ++v) g[v] = inner ? dv<R, SP>(Pn[v] - Pp[v], dx, r, &fo) : R(0);
   // lane 0's back neighbour is itself (0 / 0): its gradient reaches no updated cell
   if constexpr (SP) { if ((threadIdx.x & 31) != 0) *oor |= fo; }
 }
 
-// Limited cell gradient from the back and front face gradients (R:497-506):
-//   gc = 0; if (gb != 0) gc += 0.5*(phi(gf/gb)*gb); if (gf != 0) gc += 0.5*(phi(gb/gf)*gf).
-// For minmod, phi(r) = max(0, min(1, r)): with finite gb, gf of opposite signs or
-// a zero the two terms are signed zeros and gc = +0; with equal signs the ratio
-// whose numerator is the smaller magnitude is the only one below 1, the other
-// term is exactly 0.5*g.  So one division gives the reference's bits.
-template <typename R>
-__device__ __forceinline__ R limited_one(int lim, R gb, R gf) {
-  const R h = R(0.5), one = R(1), zero = R(0);
-  if (lim == 0) {
-    if (gb == zero || gf == zero || ((gb > zero) != (gf > zero))) return zero;
-    const bool fsmall = fabs(gf) < fabs(gb);
-    const R r = fsmall ? Ar<R>::quo(gf, gb) : Ar<R>::quo(gb, gf);
-    const R t1 = fsmall ? h * (r * gb) : h * (one * gb);
-    const R t2 = fsmall ? h * (one * gf) : h * (r * gf);
-    return (zero + t1) + t2;
-  }
-  R gc = zero;
-  if (gb != zero) gc += h * (limiter<R>(lim, Ar<R>::quo(gf, gb)) * gb);
-  if (gf != zero) gc += h * (limiter<R>(lim, Ar<R>::quo(gb, gf)) * gf);
-  return gc;
+// Limited cell gradient from the back and front face gradients (R:497-506).
+template <typename R, bool SP = false>
+__device__ __forceinline__ R limited_one(int lim, R gb, R gf, unsigned* oor = nullptr) {
+  return limited_slope<R, false, SP>(lim, gb, gf, oor);
 }
 
 // Variable 0 (the volume) has Phi = U0/U0 = 1 on every cell of a
 // single-environment mesh, so its face gradients are zero and its limited
 // gradient is +0; only variables 1..3 are computed.
-template <typename R>
-__device__ __forceinline__ void limited_grad(int lim, const R gb[4], const R gf[4], R G[4]) {
+template <typename R, bool SP = false>
+__device__ __forceinline__ void limited_grad(int lim, const R gb[4], const R gf[4], R G[4], unsigned* oor = nullptr) {
   G[0] = 0;
 #pragma unroll
-  for (int v = 1; v < 4; ++v) G[v] = limited_one<R>(lim, gb[v], gf[v]);
+  for (int v = 1; v < 4; ++v) G[v] = limited_one<R, SP>(lim, gb[v], gf[v], oor);
 }
 
 // Upwind face value (R:707-714): from the previous cell when u_f dx_f > 0.
@@ -404,9 +387,9 @@ __device__ __forceinline__ void cell_line(const Phys& ph, double dt, const Scala
 #pragma unroll
   for (int v = 0; v < 4; ++v) Pp[v] = __shfl_up_sync(full, P[v], 1);
   if constexpr (PB) {
-    const R r = inner ? Ar<R>::rcp((R)dx) : R(0);
+    const R r = inner ? R(1) / (R)dx : R(0);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) g[v] = inner ? Ar<R>::div(P[v] - Pp[v], (R)dx, r) : R(0);
+    for (int v = 0; v < 4; ++v) g[v] = inner ? qdiv(P[v] - Pp[v], (R)dx, r) : R(0);
   } else {
     face_grad<R, SP>(inner, (R)dx, P, Pp, g, oor);
   }
@@ -447,7 +430,10 @@ __device__ __forceinline__ void cell_line(const Phys& ph, double dt, const Scala
     for (int v = 0; v < 4; ++v)
       G[v] = flux_limiter_g<R>(lim, gr[v], g[v], P[v], infr ? Pn[v] : P[v], inner ? Pp[v] : P[v], h0, hp, hm);
   } else {
-    limited_grad<R>(lim, g, gr, G);
+    // only the gradients of lanes 1..30 reach an updated cell
+    unsigned go = 0u;
+    limited_grad<R, SP>(lim, g, gr, G, &go);
+    if constexpr (SP) { const int lane = threadIdx.x & 31; if (lane >= 1 && lane <= 30) *oor |= go; }
   }
 #pragma unroll
   for (int v = 0; v < 4; ++v) Gp[v] = __shfl_up_sync(full, G[v], 1);
@@ -528,28 +514,6 @@ __device__ __forceinline__ void dual_update(int D, R order2, R dt, double bfm, d
   ud[0] = out[0]; ud[1] = out[1]; ud[2] = out[2]; ud[3] = u3; ud[4] = out[3];
 }
 
-// One limited nodal gradient component (DualPhaseRemap.cc:736-777) from the
-// back and front differences; the terms are (0.5*phi(r))*g here, and the same
-// single-division reading of minmod applies.
-template <typename R>
-__device__ __forceinline__ R dual_limited(int lim, R gb, R gf) {
-  const R h = R(0.5), one = R(1), zero = R(0);
-  R g = zero;
-  if (lim == 0) {
-    if (!(gb == zero || gf == zero || ((gb > zero) != (gf > zero)))) {
-      const bool fsmall = fabs(gf) < fabs(gb);
-      const R r = fsmall ? Ar<R>::quo(gf, gb) : Ar<R>::quo(gb, gf);
-      const R t1 = fsmall ? h * r * gb : h * one * gb;
-      const R t2 = fsmall ? h * one * gf : h * r * gf;
-      g = (zero + t1) + t2;
-    }
-  } else {
-    if (gb != zero) g += h * limiter<R>(lim, Ar<R>::quo(gf, gb)) * gb;
-    if (gf != zero) g += h * limiter<R>(lim, Ar<R>::quo(gb, gf)) * gf;
-  }
-  return g;
-}
-
 // Inputs of one lane (one node of a line along d).
 struct NodeIn {
   double vh[3];    // Lagrange velocity
@@ -591,7 +555,7 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
 #pragma unroll
       for (int c = 0; c < 5; ++c) ud[c] = in.ud[c];
       if (updated) {
-        const R m = (R)ud[3], rm = Ar<R>::rcp(m);
+        const R m = (R)ud[3], rm = rc<R, SP>(m, oor);
         P[0] = dv<R, SP>((R)ud[0], m, rm, oor); P[1] = dv<R, SP>((R)ud[1], m, rm, oor);
         P[2] = dv<R, SP>((R)ud[2], m, rm, oor); P[3] = dv<R, SP>((R)ud[4], m, rm, oor);
       } else {
@@ -607,11 +571,11 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
   const double xm = __shfl_up_sync(full, x, 1), xp = __shfl_down_sync(full, x, 1);
   if (grad_on) {
     // front difference quotient of this node = back difference quotient of the next
-    const R hf = (R)(xp - x), rf = Ar<R>::rcp(hf);
     R gf[3], gb[3];
     // speculative quotients count only where they are used: a valid node
     // whose next node is valid and in this warp (the last lane divides by 0)
     unsigned gfo = 0u;
+    const R hf = (R)(xp - x), rf = rc<R, SP>(hf, &gfo);
 #pragma unroll
     for (int c = 0; c < 3; ++c) gf[c] = dv<R, SP>(Pp[c] - P[c], hf, rf, &gfo);
     if constexpr (SP) {
@@ -639,8 +603,10 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
         for (int c = 0; c < 3; ++c) G[c] = flux_limiter_g<R>(lim, gf[c], gb[c], P[c], Pp[c], Pm[c], h0, hpl, hmo);
       }
     } else if (valid && inner) {
+      unsigned go = 0u;                               // lanes 1..30: what reaches an updated node
 #pragma unroll
-      for (int c = 0; c < 3; ++c) G[c] = dual_limited<R>(lim, gb[c], gf[c]);
+      for (int c = 0; c < 3; ++c) G[c] = limited_slope<R, true, SP>(lim, gb[c], gf[c], &go);
+      if constexpr (SP) { const int lane = threadIdx.x & 31; if (lane >= 1 && lane <= 30) *oor |= go; }
     }
   }
   R Gm[3], Gp[3];
@@ -657,7 +623,7 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
     D3 u;
     double rm = 0.;
     if (m != 0.) {
-      rm = 1.0 / m;
+      rm = rc<double, SP>(m, oor);
       u = d3(dv<double, SP>(ud[0], m, rm, oor), dv<double, SP>(ud[1], m, rm, oor), dv<double, SP>(ud[2], m, rm, oor));
     } else {
       u = d3(in.vh[0], in.vh[1], in.vh[2]);

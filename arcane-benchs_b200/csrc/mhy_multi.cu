@@ -63,14 +63,14 @@ __device__ __forceinline__ void face_values_env(const Phys& ph, int lim, bool in
                xpz = __shfl_up_sync(full, in.xc[2], 1);
   const double dx = inner ? dot(d3(in.xc[0], in.xc[1], in.xc[2]) - d3(xpx, xpy, xpz), d3(in.n[0], in.n[1], in.n[2]))
                           : 0.;
-  const R dxR = (R)dx, rdx = inner ? Ar<R>::rcp(dxR) : R(0);
+  unsigned fo = 0u, go = 0u;
+  const R dxR = (R)dx, rdx = inner ? rc<R, SP>(dxR, &fo) : R(0);
   R G[NV], Pp[NV];
   R h0 = R(0), hm = R(0), hp = R(0);
   if constexpr (GL) {
     const double hb = __shfl_up_sync(full, in.h, 1), hn = __shfl_down_sync(full, in.h, 1);
     h0 = (R)in.h; hm = (R)(inner ? hb : in.h); hp = (R)(infr ? hn : in.h);
   }
-  unsigned fo = 0u;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     Pp[v] = __shfl_up_sync(full, P[v], 1);
@@ -81,11 +81,16 @@ __device__ __forceinline__ void face_values_env(const Phys& ph, int lim, bool in
       G[v] = lim < 3 ? limited_one<R>(lim, g, gr)
                      : flux_limiter_g<R>(lim, gr, g, P[v], infr ? Pn : P[v], inner ? Pp[v] : P[v], h0, hp, hm);
     } else {
-      G[v] = limited_one<R>(lim, g, gr);
+      G[v] = limited_one<R, SP>(lim, g, gr, &go);
     }
   }
-  // lane 0's back neighbour is itself (0 / 0): its gradient reaches no updated cell
-  if constexpr (SP) { if ((threadIdx.x & 31) != 0) *oor |= fo; }
+  // lane 0's back neighbour is itself (0 / 0): its face gradient reaches no
+  // updated cell, and only the limited gradients of lanes 1..30 do
+  if constexpr (SP) {
+    const int lane = threadIdx.x & 31;
+    if (lane != 0) *oor |= fo;
+    if (lane >= 1 && lane <= 30) *oor |= go;
+  }
   const bool back = in.u * dx > 0.0;
   const R dot_xf = (R)(back ? in.db : in.df);
 #pragma unroll
@@ -202,7 +207,7 @@ __device__ __forceinline__ void cell_line_env(const Phys& ph, double dt, bool va
 #pragma unroll
           for (int k = 0; k < K; ++k) den += in.U[k];
         }
-        const R dR = (R)den, r = Ar<R>::rcp(dR);
+        const R dR = (R)den, r = rc<R, SP>(dR, oor);
 #pragma unroll
         for (int v = 0; v < NV; ++v) P[v] = dv<R, SP>((R)in.U[v], dR, r, oor);
       }
