@@ -707,8 +707,10 @@ struct mhy_batch {
   std::vector<mhy_ctx*> inst;
   CycleArgs* d_descs = nullptr;
   int4* d_work[BK_COUNT] = {};
+  int4* d_cwork = nullptr;                      // the Lagrange cell kernel's columns
   int4* d_o3work[3] = {};                       // order 3: face work tables per direction
   int4* d_fwork = nullptr;                      // schema-csts: face work table (all directions)
+  int col_order = 0;                            // and of the columns
   int order[BK_COUNT] = {};                     // work-table order of each kind (mhy_tuning.order)
   BatchPlan plan{};
   int sens = 0;
@@ -721,6 +723,8 @@ namespace {
 
 // Work table of one kernel kind: every block of every instance's grid, in
 // one of three orders (mhy_tuning.order), for the given lines per block.
+// kColumns instead of a kind: the columns of the Lagrange cell kernel.
+constexpr int kColumns = -1;
 std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int order, int lines) {
   const int n = (int)inst.size();
   std::vector<int> ids(n);
@@ -730,7 +734,13 @@ std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int or
   std::vector<std::vector<int4>> per(n);
   for (int i = 0; i < n; ++i) {
     int gx, gy, gz;
-    batch_work_shape(inst[i]->dm, kind, lines, gx, gy, gz);
+    if (kind == kColumns) {
+      size_t smem;
+      batch_column_shape(inst[i]->dm, gx, gy, smem);
+      gz = 1;
+    } else {
+      batch_work_shape(inst[i]->dm, kind, lines, gx, gy, gz);
+    }
     if (gy < 0) {                               // linear chunks of consecutive items
       for (int x = 0; x < gx; ++x) per[i].push_back(make_int4(i, x, -1, 0));
       continue;
@@ -764,6 +774,7 @@ void mhy_batch_destroy(mhy_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (int s = 0; s < 3; ++s) if (b->graph[s]) cudaGraphExecDestroy(b->graph[s]);
   for (int k = 0; k < BK_COUNT; ++k) if (b->d_work[k]) cudaFree(b->d_work[k]);
+  if (b->d_cwork) cudaFree(b->d_cwork);
   for (int d = 0; d < 3; ++d) if (b->d_o3work[d]) cudaFree(b->d_o3work[d]);
   if (b->d_fwork) cudaFree(b->d_fwork);
   if (b->d_descs) cudaFree(b->d_descs);
@@ -809,6 +820,20 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
     if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
     b->plan.work[k] = b->d_work[k];
     b->plan.nwork[k] = (int)w.size();
+  }
+  {
+    const std::vector<int4> w = build_work(b->inst, kColumns, 0, kLineWarps);
+    err = cudaMalloc(&b->d_cwork, w.size() * sizeof(int4));
+    if (err == cudaSuccess) err = cudaMemcpy(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
+    b->plan.cwork = b->d_cwork;
+    b->plan.ncwork = (int)w.size();
+    for (const mhy_ctx* c : b->inst) {
+      int blocks, segments;
+      size_t smem;
+      batch_column_shape(c->dm, blocks, segments, smem);
+      b->plan.col_smem = std::max(b->plan.col_smem, smem);
+    }
   }
   err = cudaMalloc(&b->d_descs, n * sizeof(CycleArgs));
   if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
@@ -1002,6 +1027,12 @@ int apply_tuning(mhy_batch* b, const mhy_tuning& t) {
     b->order[k] = t.order[k];
     b->plan.lines[k] = t.lines_per_block[k];
     b->plan.nwork[k] = (int)w.size();
+  }
+  if (t.order[BK_LCELLS] != b->col_order) {
+    const std::vector<int4> w = build_work(b->inst, kColumns, t.order[BK_LCELLS], kLineWarps);
+    MHY_CUDA(cudaMemcpyAsync(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
+    MHY_CUDA(cudaStreamSynchronize(b->stream));
+    b->col_order = t.order[BK_LCELLS];
   }
   for (int k = 0; k < BK_TUNE_SLOTS; ++k) b->plan.occ_pct[k] = t.occupancy_pct[k];
   for (int s = 0; s < 3; ++s)

@@ -540,18 +540,9 @@ void launch_lagrange_cells(const CycleArgs& a, cudaStream_t s) {
     auto kern = hc ? k_cyc_lagrange_cells_csts<1, true> : k_cyc_lagrange_cells_csts<1, false>;
     kern<<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p, a.st.cs, a.st.mass,
                              a.cqs, a.L, a.U[0], a.xc, a.fd, a.env, a.Vlag, linear, a.vnb, a.pf);
-  } else if (hc && !a.ph.precision) {
-    k_cyc_lagrange_cells<1, double, true><<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e,
-                                                              a.st.q, a.st.p, a.st.cs, a.st.mass, a.cqs, a.cqs32, a.L,
-                                                              a.U[0], a.xc, a.fd, a.env, a.Vlag, linear);
-  } else if (a.ph.precision)
-    k_cyc_lagrange_cells<1, float><<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q,
-                                                       a.st.p, a.st.cs, a.st.mass, a.cqs, a.cqs32, a.L, a.U[0], a.xc,
-                                                       a.fd, a.env, a.Vlag, linear);
-  else
-    k_cyc_lagrange_cells<1, double><<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q,
-                                                        a.st.p, a.st.cs, a.st.mass, a.cqs, a.cqs32, a.L, a.U[0], a.xc,
-                                                        a.fd, a.env, a.Vlag, linear);
+    return;
+  }
+  launch_cells<1>(a, s);
 }
 
 // Three sweeps d = (i + sens) % 3 (RemapADIService.cc:28-30).  U: Lagrange
@@ -723,18 +714,6 @@ __global__ void __launch_bounds__(128) k_bat_lagrange_nodes(const CycleArgs* __r
   }
 }
 
-template <typename R, bool HC = false, bool CSTS = false>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_lagrange_cells(const CycleArgs* __restrict__ D,
-                                                                                   const int4* __restrict__ W, int nw) {
-  for (int w = blockIdx.x; w < nw; w += gridDim.x) {
-    const int4 t = W[w];
-    const CycleArgs& a = D[t.x];
-    k_cyc_lagrange_cells_body<1, R, CSTS, HC>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p,
-                                              a.st.cs, a.st.mass, a.cqs, CSTS ? nullptr : a.cqs32, a.L, a.U[0], a.xc,
-                                              a.fd, a.env, a.Vlag, t.y, t.z, t.w, a.vnb, a.pf);
-  }
-}
-
 // schema-csts of every instance: the forward velocity and the Lagrangian
 // coordinates over the node tiles, then the face velocities over the face
 // work table (instance, chunk of 128 faces of all directions)
@@ -892,6 +871,12 @@ int persistent_grid(const void* kernel, int threads, size_t smem, int nwork, int
   return persistent_blocks(kernel, threads, smem, nwork, pct);
 }
 
+void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem) {
+  blocks = col_blocks(dm.nx, dm.ny);
+  segments = col_segments(dm.nx, dm.ny, dm.nz);
+  smem = col_smem(dm.nx);
+}
+
 void mark(KernelMarks* m, int kind, cudaStream_t s) {
   if (!m || m->n >= KernelMarks::kMax) return;
   cudaEventRecord(m->ev[m->n], s);
@@ -1034,16 +1019,12 @@ void launch_batch_cycle(const BatchPlan& P, int sens, cudaStream_t s, KernelMark
   if (P.K > 1) { launch_batch_cycle_env(P, sens, s, m); return; }
   launch_bat_lagrange_nodes(P, s, m);
   const bool hc = P.gl || P.pb || P.o3;   // the G limiters, pente-borne, order 3: the cell widths too
-  if (P.precision)
-    launch_persistent(k_bat_lagrange_cells<float>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  else if (P.csts && hc)
-    launch_persistent(k_bat_lagrange_cells<double, true, true>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  else if (P.csts)
-    launch_persistent(k_bat_lagrange_cells<double, false, true>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  else if (hc)
-    launch_persistent(k_bat_lagrange_cells<double, true>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  else
-    launch_persistent(k_bat_lagrange_cells<double>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+  if (P.csts || P.precision) {
+    auto kern = P.precision ? k_bat_lagrange_cells<1, float, false, false>
+                            : (hc ? k_bat_lagrange_cells<1, double, true, true> : k_bat_lagrange_cells<1, double, false, true>);
+    launch_persistent(kern, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+  } else if (hc) launch_bat_columns(k_bat_lagrange_columns<1, true>, P, s, m);
+  else launch_bat_columns(k_bat_lagrange_columns<1, false>, P, s, m);
   launch_bat_csts_forward(P, s);   // PrepareRemap.cc:456, then the face velocities
   if (P.precision) bat_sweeps<float, false>(P, sens, s, m);
   else if (P.gl) bat_sweeps<double, true>(P, sens, s, m);

@@ -147,43 +147,78 @@ __device__ __forceinline__ R limiter(int id, R r, unsigned* oor = nullptr) {
 // For minmod, phi(r) = max(0, min(1, r)): with finite gb, gf of opposite signs or
 // a zero the two terms are signed zeros and g = +0; with equal signs the ratio
 // whose numerator is the smaller magnitude is the only one below 1, the other
-// term is exactly 0.5 g.  So one division gives the reference's bits.  For
-// superBee and vanLeer the speculative form takes the same g = +0 for
-// differences of opposite signs or a zero, and raises *oor for differences of
-// 1e150 and more, infinities and NaN, whose terms may be other than zero.
-template <typename R, bool DUAL, bool SP>
-__device__ __forceinline__ R limited_slope(int lim, R gb, R gf, unsigned* oor) {
+// term is exactly 0.5 g.  So one division gives the reference's bits.
+template <typename R, bool DUAL>
+__device__ __forceinline__ R limited_slope(int lim, R gb, R gf) {
   const R h = R(0.5), one = R(1), zero = R(0);
   if (lim == 0) {
-    if constexpr (sizeof(R) == 8 && SP) {
-      const bool live = !(gb == zero || gf == zero || ((gb > zero) != (gf > zero)));
-      const bool fsmall = fabs(gf) < fabs(gb);
-      const R num = fsmall ? gf : gb, den = fsmall ? gb : gf;
-      unsigned bad = 0u;
-      const R r = quo_fast(num, den, bad);
-      if (live) *oor |= bad;
-      const R t1 = DUAL ? h * r * den : h * (r * den), t2 = DUAL ? h * one * num : h * (one * num);
-      return live ? (zero + t1) + t2 : zero;
-    } else {
-      if (gb == zero || gf == zero || ((gb > zero) != (gf > zero))) return zero;
-      const bool fsmall = fabs(gf) < fabs(gb);
-      const R r = fsmall ? qu<R, false>(gf, gb, nullptr) : qu<R, false>(gb, gf, nullptr);
-      const R t1 = fsmall ? (DUAL ? h * r * gb : h * (r * gb)) : (DUAL ? h * one * gb : h * (one * gb));
-      const R t2 = fsmall ? (DUAL ? h * one * gf : h * (one * gf)) : (DUAL ? h * r * gf : h * (r * gf));
-      return (zero + t1) + t2;
-    }
+    if (gb == zero || gf == zero || ((gb > zero) != (gf > zero))) return zero;
+    const bool fsmall = fabs(gf) < fabs(gb);
+    const R r = fsmall ? qu<R, false>(gf, gb, nullptr) : qu<R, false>(gb, gf, nullptr);
+    const R t1 = fsmall ? (DUAL ? h * r * gb : h * (r * gb)) : (DUAL ? h * one * gb : h * (one * gb));
+    const R t2 = fsmall ? (DUAL ? h * one * gf : h * (one * gf)) : (DUAL ? h * r * gf : h * (r * gf));
+    return (zero + t1) + t2;
   }
+  R g = zero;
+  if (gb != zero) { const R p = limiter<R>(lim, qu<R, false>(gf, gb, nullptr)); g += DUAL ? h * p * gb : h * (p * gb); }
+  if (gf != zero) { const R p = limiter<R>(lim, qu<R, false>(gb, gf, nullptr)); g += DUAL ? h * p * gf : h * (p * gf); }
+  return g;
+}
+
+// NV of them.  The speculative form takes zero where a pair has opposite signs
+// or a zero.  For superBee and vanLeer it also raises *oor for differences of
+// 1e150 and more, infinities and NaN, whose terms may be other than zero at
+// opposite signs.  Nothing is skipped where there is nothing to limit, so that
+// the slopes overlap.
+template <int NV, typename R, bool DUAL, bool SP>
+__device__ __forceinline__ void limited_slopes(int lim, const R* gb, const R* gf, R* G, unsigned* oor) {
+  const R h = R(0.5), one = R(1), zero = R(0);
   if constexpr (sizeof(R) == 8 && SP) {
-    if (!(fabs(gb) < 1e150 && fabs(gf) < 1e150)) *oor = 1u;
-    if (lim < 0 || (gb <= zero && gf >= zero) || (gb >= zero && gf <= zero)) return zero;   // lim < 0: order 1
-    const R rb = quo_fast(gf, gb, *oor), rf = quo_fast(gb, gf, *oor);
-    const R pb = limiter<R, true>(lim, rb, oor), pf = limiter<R, true>(lim, rf, oor);
-    return (zero + (DUAL ? h * pb * gb : h * (pb * gb))) + (DUAL ? h * pf * gf : h * (pf * gf));
+    bool live[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      live[v] = !((gb[v] <= zero && gf[v] >= zero) || (gb[v] >= zero && gf[v] <= zero));
+      G[v] = zero;
+    }
+    if (lim != 0) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        if (!(fabs(gb[v]) < 1e150 && fabs(gf[v]) < 1e150)) *oor = 1u;
+    }
+    if (lim >= 0) {                                          // lim < 0: order 1
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        unsigned bad = 0u;
+        R g;
+        if (lim == 0) {
+          const bool fsmall = fabs(gf[v]) < fabs(gb[v]);
+          const R num = fsmall ? gf[v] : gb[v], den = fsmall ? gb[v] : gf[v];
+          const R r = quo_fast(num, den, bad);
+          const R t1 = DUAL ? h * r * den : h * (r * den), t2 = DUAL ? h * one * num : h * (one * num);
+          g = (zero + t1) + t2;
+        } else {
+          const R rb = quo_fast(gf[v], gb[v], bad), rf = quo_fast(gb[v], gf[v], bad);
+          const R pb = limiter<R, true>(lim, rb, &bad), pf = limiter<R, true>(lim, rf, &bad);
+          g = (zero + (DUAL ? h * pb * gb[v] : h * (pb * gb[v]))) + (DUAL ? h * pf * gf[v] : h * (pf * gf[v]));
+        }
+        if (live[v]) { G[v] = g; *oor |= bad; }
+      }
+    }
   } else {
-    R g = zero;
-    if (gb != zero) { const R p = limiter<R>(lim, qu<R, false>(gf, gb, nullptr)); g += DUAL ? h * p * gb : h * (p * gb); }
-    if (gf != zero) { const R p = limiter<R>(lim, qu<R, false>(gb, gf, nullptr)); g += DUAL ? h * p * gf : h * (p * gf); }
-    return g;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) G[v] = limited_slope<R, DUAL>(lim, gb[v], gf[v]);
+  }
+}
+
+// V^(1./3.) (mhy_pow_third.h); the speculative form raises *oor for a V that is
+// not a positive normal number.
+template <bool SP>
+__device__ __forceinline__ double pow_third_of(double v, unsigned* oor) {
+  if constexpr (SP) {
+    if (!(v >= 0x1p-1022 && v < 0x1p+1023)) *oor = 1u;
+    return pow_third_normal(v, 0, [&](double x, double y) { return quo_fast(x, y, *oor); });
+  } else {
+    return pow_third(v);
   }
 }
 
@@ -204,14 +239,15 @@ __device__ __forceinline__ void eos_init(int kind, double g, double pinf, double
 }
 
 // compute_eint, mahyco/src/MahycoModule.cc:1630-1654; ir = 1.0/r and irn = 1.0/rn given.
+template <bool SP = false>
 __device__ __forceinline__ double compute_eint(bool pc, double g, double qn, double q, double ir, double irn,
-                                               double r, double p, double en) {
+                                               double r, double p, double en, unsigned* oor = nullptr) {
   double pseudo = 0.;
   if (pc && ((qn + q) * (ir - irn) < 0.)) pseudo = 0.5 * (q + qn);
   if (!pc && (q * (ir - irn) < 0.)) pseudo = q;
   double denom = 1 + 0.5 * (g - 1.0) * r * (ir - irn);
   double numer = en - (0.5 * p + pseudo) * (ir - irn);
-  return numer / denom;
+  return qu<double, SP>(numer, denom, oor);
 }
 
 // updateEnergyAndPressurebyNewton without schema-csts, MahycoModule.cc:1482-1535:
@@ -243,11 +279,12 @@ __device__ __forceinline__ double newton_eint(bool pc, int kind, double g, doubl
 
 // The Lagrange energy update of one environment cell: the closed form of
 // updateEnergyAndPressureforGP, or the Newton iterations when with-newton is set.
+template <bool SP = false>
 __device__ __forceinline__ double energy_update(bool newton, bool pc, int kind, double g, double pinf, double epsilon,
                                                 double qn, double q, double ir, double irn, double r, double p,
-                                                double en) {
+                                                double en, unsigned* oor = nullptr) {
   if (newton) return newton_eint(pc, kind, g, pinf, epsilon, qn, q, ir, irn, r, p, en);
-  return compute_eint(pc, g, qn, q, ir, irn, r, p, en);
+  return compute_eint<SP>(pc, g, qn, q, ir, irn, r, p, en, oor);
 }
 
 // Corner vectors (CQS) of a hexahedron, mahyco/src/MahycoModule.cc:2195-2258,

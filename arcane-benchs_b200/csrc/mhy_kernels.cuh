@@ -160,6 +160,9 @@ struct BatchPlan {
   int pb;                       // every instance takes projection-pente-borne (FP64): the PB cell sweeps
   int o3;                       // every instance takes order 3 (FP64): face values, then the O3 cell sweeps
   int csts;                     // every instance takes schema-csts (FP64)
+  const int4* cwork;            // the Lagrange cell kernel's columns (instance, chunk, segment); not schema-csts
+  int ncwork;
+  size_t col_smem;              // its shared memory, the largest instance's
   const int4* fwork;            // schema-csts: face work table (instance, chunk of 128 faces of all directions)
   int nfwork;
   const int4* o3work[3];        // order 3: face work tables (instance, chunk of 128 faces) per direction
@@ -175,6 +178,9 @@ struct KernelMarks {
   int n;
 };
 void batch_work_shape(const Dims& dm, int kind, int lines, int& gx, int& gy, int& gz);
+void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem);
+// Dynamic shared memory above the default 48 KB needs an opt-in per kernel and device.
+void smem_opt_in(const void* kernel, size_t bytes);
 // Records an event after a launch (autotuning): slot `kind` of the marks.
 void mark(KernelMarks* m, int kind, cudaStream_t s);
 // Batched cycle helpers: the resident-block grid of a persistent kernel, the

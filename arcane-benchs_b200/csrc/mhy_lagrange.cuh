@@ -114,17 +114,19 @@ __device__ __forceinline__ void corner_vectors(const Vec3<T> x[8], Finish&& fini
 }
 
 // Remap face data from a cell's nodes (PrepareRemap.cc:41-55, 105-117;
-// RemapADIService.cc:710): for the low face of each direction (an inner
-// face) |A| along d, u_f and (x_f - x_c).n0 with this cell as the next cell;
-// for the high face (an inner face) (x_f - x_c).n0 with this cell as the
+// RemapADIService.cc:710): for the low face of each direction |A| along d, u_f and (x_f - x_c).n0 with this cell as the next cell;
+// for the high face (x_f - x_c).n0 with this cell as the
 // previous one.  Face node order: X (0,3,7,4), Y (0,1,5,4), Z (0,1,2,3) low;
 // X (1,2,6,5), Y (3,2,6,7), Z (4,5,6,7) high, in SN_trigo cell-node numbers.
+// In FP64 the values of boundary faces are written too and read by nobody:
+// without a branch the faces' arithmetic overlaps the chain of the thermodynamics.
 // T = float takes x relative to the cell centre (xc = 0).  HC: also the cell
 // widths along each direction into fd.h (order 3 and the generalised limiters).
-template <typename T, bool HC = false>
+// nlo(d), nhi(d): the normals of the low and high face of direction d; vn(a):
+// the Lagrange velocity of cell node a.
+template <typename T, bool HC, typename Nlo, typename Nhi, typename Vn>
 __device__ __forceinline__ void face_data(const Dims& dm, int i, int j, int k, const Vec3<T> x[8], Vec3<T> xc,
-                                          const double* __restrict__ n0, const double* __restrict__ vh,
-                                          const FaceData& fd) {
+                                          const FaceData& fd, Nlo&& nlo, Nhi&& nhi, Vn&& vn) {
   const T q = T(.25);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -133,9 +135,9 @@ __device__ __forceinline__ void face_data(const Dims& dm, int i, int j, int k, c
     const int lo[3][4] = {{0, 3, 7, 4}, {0, 1, 5, 4}, {0, 1, 2, 3}};
     const int hi[3][4] = {{1, 2, 6, 5}, {3, 2, 6, 7}, {4, 5, 6, 7}};
     const long long off = d == 0 ? 0 : (d == 1 ? dm.Fx : dm.Fx + dm.Fy);
-    if (id > 0) {
+    if (sizeof(T) == 8 || id > 0) {
       const long long f = dm.fid(d, i, j, k);
-      const D3 nrm = d3(n0[f], n0[dm.F + f], n0[2 * dm.F + f]);
+      const D3 nrm = nlo(d);
       const Vec3<T> nr = Vec3<T>{(T)nrm.x, (T)nrm.y, (T)nrm.z};
       const Vec3<T> a0 = x[lo[d][0]], a1 = x[lo[d][1]], a2 = x[lo[d][2]], a3 = x[lo[d][3]];
       Vec3<T> xf = Vec3<T>{0, 0, 0};
@@ -143,9 +145,7 @@ __device__ __forceinline__ void face_data(const Dims& dm, int i, int j, int k, c
       D3 vs = d3(0., 0., 0.);
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int a = lo[d][b];
-        const long long nn = dm.nid(i + kCellNodeOff[a][0], j + kCellNodeOff[a][1], k + kCellNodeOff[a][2]);
-        vs = vs + d3(vh[nn], vh[dm.N + nn], vh[2 * dm.N + nn]);
+        vs = vs + vn(lo[d][b]);
       }
       const Vec3<T> cr = T(0.5) * cross(a2 - a0, a3 - a1);
       double A = fabs((double)comp(cr, d));
@@ -154,15 +154,16 @@ __device__ __forceinline__ void face_data(const Dims& dm, int i, int j, int k, c
       fd.A[d][t] = A;
       fd.u[d][t] = dot(.25 * vs, nrm);
       fd.df[d][t] = (double)dot(xf - xc, nr);
-      if constexpr (HC) hsum += norm2(xf - xc);
+      if constexpr (HC) { if (id > 0) hsum += norm2(xf - xc); }
     }
-    if (id + 1 < dm.ncd(d)) {
+    if (sizeof(T) == 8 || id + 1 < dm.ncd(d)) {
       const long long f = dm.fid(d, i + (d == 0), j + (d == 1), k + (d == 2));
-      const Vec3<T> nr = Vec3<T>{(T)n0[f], (T)n0[dm.F + f], (T)n0[2 * dm.F + f]};
+      const D3 nrm = nhi(d);
+      const Vec3<T> nr = Vec3<T>{(T)nrm.x, (T)nrm.y, (T)nrm.z};
       Vec3<T> xf = Vec3<T>{0, 0, 0};
       xf = xf + q * x[hi[d][0]]; xf = xf + q * x[hi[d][1]]; xf = xf + q * x[hi[d][2]]; xf = xf + q * x[hi[d][3]];
       fd.db[d][f - off] = (double)dot(xf - xc, nr);
-      if constexpr (HC) hsum += norm2(xf - xc);
+      if constexpr (HC) { if (id + 1 < dm.ncd(d)) hsum += norm2(xf - xc); }
     }
     if constexpr (HC) fd.h[d * dm.C + dm.cid(i, j, k)] = hsum;
   }
@@ -208,6 +209,55 @@ __device__ __forceinline__ double csts_eint(const Phys& ph, double g, int eos, d
   return e;
 }
 
+// Lagrange thermodynamics of a cell of one environment (MahycoModule.cc:1331-1426
+// updateDensity, :454-578 computeArtificialViscosity, :1659-1770
+// updateEnergyAndPressureforGP): the characteristic length, density,
+// pseudo-viscosity and energy.  SP: the quotients of mhy_quot.h, without a
+// branch, so that this chain of a dozen dependent quotients overlaps the face
+// data; *oor is raised where they may differ and the cell is done again by
+// thermo_one_exact.  Measured on B200 with plain quotients -> with these: cell
+// kernel of Sedov 128^3 377 -> 323 us in FP64, 230 -> 219 us in the mixed form.
+struct ThermoIn { double V, inv_dt, rn, m, cs, p, q, e; };
+struct ThermoOut { double L, nd, qn, en, pf; };
+template <bool CSTS, bool F32, bool SP>
+__device__ __forceinline__ ThermoOut thermo_one(const Phys& ph, const ThermoIn& in, double Lface, double cn1, double cn,
+                                                double cdn, double con, unsigned* oor) {
+  ThermoOut o;
+  o.pf = 0.;
+  // racine-cubique-volume: the project cube root (the reference's bits) in
+  // FP64; the mixed form takes CUDA's FP32 cube root of the FP64 volume (L
+  // feeds the viscosity and the CFL bound only)
+  if (ph.lc_mode == 0) {
+    if constexpr (F32) o.L = (double)cbrtf((float)in.V);
+    else o.L = pow_third_of<SP>(in.V, oor);
+  } else {
+    o.L = Lface;
+  }
+  const double nd = qu<double, SP>(in.m, in.V, oor);
+  const double irn = rc<double, SP>(in.rn, oor), ind = rc<double, SP>(nd, oor);
+  const double tau = 0.5 * (irn + ind);
+  const double itau = rc<double, SP>(tau, oor);
+  const double du = dv<double, SP>(in.inv_dt * (ind - irn), tau, itau, oor);
+  double qn = 0.;
+  const double g = ph.gamma;
+  if (du < 0.0) qn = itau * (-0.5 * o.L * in.cs * du + (g + 1) / 2.0 * o.L * o.L * du * du);
+  o.nd = nd;
+  o.qn = qn;
+  if constexpr (CSTS)
+    o.en = csts_eint(ph, g, ph.eos, ph.pinf, cn1, cn, cdn, con, in.e, nd, in.m, in.p, in.q, qn, o.pf);
+  else if constexpr (SP)   // Newton takes the exact form
+    o.en = compute_eint<true>(ph.pseudo_centree != 0, g, in.q, qn, ind, irn, nd, in.p, in.e, oor);
+  else
+    o.en = energy_update(ph.with_newton != 0, ph.pseudo_centree != 0, ph.eos, g, ph.pinf, ph.threshold, in.q, qn, ind,
+                         irn, nd, in.p, in.e);
+  return o;
+}
+template <bool CSTS, bool F32>
+__device__ __noinline__ ThermoOut thermo_one_exact(Phys ph, ThermoIn in, double Lface, double cn1, double cn, double cdn,
+                                                   double con) {
+  return thermo_one<CSTS, F32, false>(ph, in, Lface, cn1, cn, cdn, con, nullptr);
+}
+
 // Lagrange thermodynamics of a mesh with K > 1 environments, then the remap
 // variables (MahycoModule.cc:1331-1426 updateDensity, :454-578
 // computeArtificialViscosity, :1659-1770 updateEnergyAndPressureforGP,
@@ -226,22 +276,22 @@ __device__ __forceinline__ double csts_eint(const Phys& ph, double g, int eos, d
 // global p + q the forward step reads (MahycoModule.cc:792-831): a pure
 // cell's p_n or Newton pressure plus its q, a mixed cell's mean p_n plus
 // sum_k f_k q_k (MahycoModule.cc:454-578).
-template <int K, bool CSTS = false>
-__device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const Scalars* S, const EnvState& env, int c,
-                                                    int C, double V, double Lc, double* __restrict__ rho,
-                                                    const double* __restrict__ e, const double* __restrict__ q,
-                                                    const double* __restrict__ p, const double* __restrict__ cs,
-                                                    const double* __restrict__ mass, double* __restrict__ U,
+// rn: the density before the step.  SP: the quotients of mhy_quot.h (see
+// thermo_one); where *oor is raised the cell is done again by
+// lagrange_thermo_env_exact, which writes all of it anew.
+template <int K, bool CSTS, bool SP>
+__device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const EnvState& env, int c, int C,
+                                                    const ThermoIn& in, double Lc, double* __restrict__ rho,
+                                                    double* __restrict__ U,
                                                     double* __restrict__ Vlag, double* __restrict__ pbphi,
-                                                    const double* cssum = nullptr, double* __restrict__ pf = nullptr) {
+                                                    const double* cssum, double* __restrict__ pf, unsigned* oor) {
   constexpr int NV = 3 * K + 1;
-  const double inv_deltat = S->inv_dt;
-  const double rn = rho[c];
-  const double nd = mass[c] / V;
-  const double irn = 1.0 / rn, ind = 1.0 / nd;
+  const double V = in.V;
+  const double nd = qu<double, SP>(in.m, V, oor);
+  const double irn = rc<double, SP>(in.rn, oor), ind = rc<double, SP>(nd, oor);
   const double tau = 0.5 * (irn + ind);
-  const double itau = 1. / tau;
-  const double du = qdiv(inv_deltat * (ind - irn), tau, itau);
+  const double itau = rc<double, SP>(tau, oor);
+  const double du = dv<double, SP>(in.inv_dt * (ind - irn), tau, itau, oor);
   const uint32_t mk = env.mask[c];
   const bool pc = ph.pseudo_centree != 0;
   double u[NV];
@@ -251,16 +301,17 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const Scalar
     const int ke = __ffs(mk) - 1;
     const double g = env.gamma[ke];
     double qn = 0.;
-    if (du < 0.0) qn = itau * (-0.5 * Lc * cs[c] * du + (g + 1) / 2.0 * Lc * Lc * du * du);
+    if (du < 0.0) qn = itau * (-0.5 * Lc * in.cs * du + (g + 1) / 2.0 * Lc * Lc * du * du);
     double en;
     if constexpr (CSTS) {
       double pforward;
-      en = csts_eint(ph, g, env.eos[ke], env.pinf[ke], cssum[0], cssum[1], cssum[2], cssum[3], e[c], nd, mass[c],
-                     p[c], q[c], qn, pforward);
+      en = csts_eint(ph, g, env.eos[ke], env.pinf[ke], cssum[0], cssum[1], cssum[2], cssum[3], in.e, nd, in.m,
+                     in.p, in.q, qn, pforward);
       pf[c] = pforward + qn;
     } else {
-      en = energy_update(ph.with_newton != 0, pc, env.eos[ke], g, env.pinf[ke], ph.threshold, q[c], qn, ind, irn, nd,
-                         p[c], e[c]);
+      en = SP ? compute_eint<SP>(pc, g, in.q, qn, ind, irn, nd, in.p, in.e, oor)
+              : energy_update(ph.with_newton != 0, pc, env.eos[ke], g, env.pinf[ke], ph.threshold, in.q, qn, ind, irn,
+                              nd, in.p, in.e);
     }
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -271,19 +322,19 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const Scalar
       pbphi[3 * K * C + c] = qn;
     }
   } else {
-    const double csc = cs[c];
+    const double csc = in.cs;
     double qg = 0.;                                              // the mixed cell's pseudo-viscosity sum_k f_k q_k
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (!(mk >> k & 1)) continue;
       const int o = k * C + c;
       const double vk = env.f[o] * V;
-      const double rk = env.m[o] / vk;
-      const double irnk = 1.0 / env.rho[o], irk = 1.0 / rk;
+      const double rk = qu<double, SP>(env.m[o], vk, oor);
+      const double irnk = rc<double, SP>(env.rho[o], oor), irk = rc<double, SP>(rk, oor);
       const double tauk = 0.5 * (irnk + irk);
       const double g = env.gamma[k];
       double qk = 0.;
-      if (du < 0.0) qk = 1. / tauk * (-0.5 * Lc * csc * du + (g + 1) / 2.0 * Lc * Lc * du * du);
+      if (du < 0.0) qk = rc<double, SP>(tauk, oor) * (-0.5 * Lc * csc * du + (g + 1) / 2.0 * Lc * Lc * du * du);
       double ek;
       if constexpr (CSTS) {
         double pk_unused;
@@ -291,8 +342,9 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const Scalar
                        env.p[o], env.q[o], qk, pk_unused);
         qg += qk * env.f[o];
       } else {
-        ek = energy_update(ph.with_newton != 0, pc, env.eos[k], g, env.pinf[k], ph.threshold, env.q[o], qk, irk, irnk,
-                           rk, env.p[o], env.e[o]);
+        ek = SP ? compute_eint<SP>(pc, g, env.q[o], qk, irk, irnk, rk, env.p[o], env.e[o], oor)
+                : energy_update(ph.with_newton != 0, pc, env.eos[k], g, env.pinf[k], ph.threshold, env.q[o], qk, irk,
+                                irnk, rk, env.p[o], env.e[o]);
       }
       u[k] = vk;
       u[K + k] = vk * rk;
@@ -302,14 +354,65 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const Scalar
         pbphi[o] = env.f[o]; pbphi[K * C + o] = rk; pbphi[2 * K * C + o] = ek; pbphi[3 * K * C + c] = qk;
       }
     }
-    if constexpr (CSTS) pf[c] = p[c] + qg;                      // the mean p_n: no EOS runs before the forward step
+    if constexpr (CSTS) pf[c] = in.p + qg;                      // the mean p_n: no EOS runs before the forward step
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) U[v * C + c] = u[v];
   Vlag[c] = V;
   rho[c] = nd;
 }
+template <int K, bool CSTS>
+__device__ __noinline__ void lagrange_thermo_env_exact(Phys ph, EnvState env, int c, int C, ThermoIn in, double Lc,
+    double* rho, double* U, double* Vlag, double* pbphi, double cn1, double cn, double cdn, double con, double* pf) {
+  const double cssum[4] = {cn1, cn, cdn, con};
+  lagrange_thermo_env<K, CSTS, false>(ph, env, c, C, in, Lc, rho, U, Vlag, pbphi, cssum, pf, nullptr);
+}
 
+// The characteristic length and the thermodynamics of a cell, then its remap
+// variables, whichever number of environments.  Lface: the length of
+// faces-opposees (used when lc_mode is 1).
+template <int K, bool CSTS, bool F32>
+__device__ __forceinline__ void cell_thermo(const Phys& ph, const EnvState& env, const FaceData& fd, int c, int C,
+                                            const ThermoIn& in, double Lface, double* __restrict__ rho,
+                                            double* __restrict__ L, double* __restrict__ U, double* __restrict__ Vlag,
+                                            double cn1, double cn, double cdn, double con, double* __restrict__ pf) {
+  unsigned oor = ph.with_newton && !CSTS ? 1u : 0u;   // Newton iterates with plain quotients
+  if constexpr (K == 1) {
+    ThermoOut t = thermo_one<CSTS, F32, true>(ph, in, Lface, cn1, cn, cdn, con, &oor);
+    if (oor) t = thermo_one_exact<CSTS, F32>(ph, in, Lface, cn1, cn, cdn, con);
+    L[c] = t.L;
+    if constexpr (CSTS) pf[c] = t.pf + t.qn;                      // the forward force's p + q (q: this cycle's)
+    U[c] = in.V;
+    U[C + c] = in.V * t.nd;
+    U[2 * C + c] = in.V * t.nd * t.en;
+    U[3 * C + c] = in.V * t.qn;
+    if (fd.pbphi) { fd.pbphi[c] = t.nd; fd.pbphi[C + c] = t.en; fd.pbphi[2 * C + c] = t.qn; }
+  } else {
+    double Lc = Lface;
+    if (ph.lc_mode == 0) {
+      if constexpr (F32) Lc = (double)cbrtf((float)in.V);
+      else {
+        unsigned lo = 0u;
+        Lc = pow_third_of<true>(in.V, &lo);
+        if (lo) Lc = pow_third(in.V);
+      }
+    }
+    L[c] = Lc;
+    const double cssum[4] = {cn1, cn, cdn, con};
+    if (!oor)
+      lagrange_thermo_env<K, CSTS, true>(ph, env, c, C, in, Lc, rho, U, Vlag, fd.pbphi, cssum, pf, &oor);
+    if (oor)
+      lagrange_thermo_env_exact<K, CSTS>(ph, env, c, C, in, Lc, rho, U, Vlag, fd.pbphi, cn1, cn, cdn, con, pf);
+  }
+}
+
+// faces-opposees: the length from the distances of opposite face centres.
+__device__ __forceinline__ double face_length(const D3 x[8]) {
+  D3 fc[6];
+  face_centres(x, fc);
+  const double d1 = norm2(fc[0] - fc[3]), d2 = norm2(fc[2] - fc[5]), d3_ = norm2(fc[1] - fc[4]);
+  return (d1 * d2 * d3_) / (d1 * d2 + d1 * d3_ + d2 * d3_);
+}
 
 // CSTS (schema-csts, FP64 only): vnb = the backward node velocity of this
 // cycle, pf = the pressure plus pseudo-viscosity of the forward step.
@@ -386,60 +489,28 @@ __device__ __forceinline__ void k_cyc_lagrange_cells_body(Dims dm, const Scalars
     }
   }
   V *= 1. / 3;
-  double Lc;
-  // racine-cubique-volume: the project cube root (the reference's bits) in
-  // FP64; the mixed form takes CUDA's FP32 cube root of the FP64 volume (L
-  // feeds the viscosity and the CFL bound only)
-  if (ph.lc_mode == 0) {
-    if constexpr (F32) Lc = (double)cbrtf((float)V);
-    else Lc = pow_third(V);
-  } else {
-    D3 fc[6];
+  double Lc = 0.;
+  if (ph.lc_mode != 0) {
     if constexpr (F32) {
       D3 xx[8];
 #pragma unroll
       for (int a = 0; a < 8; ++a) xx[a] = d3(xr[a].x, xr[a].y, xr[a].z);
-      face_centres(xx, fc);
+      Lc = face_length(xx);
     } else {
-      face_centres(x, fc);
+      Lc = face_length(x);
     }
-    const double d1 = norm2(fc[0] - fc[3]), d2 = norm2(fc[2] - fc[5]), d3_ = norm2(fc[1] - fc[4]);
-    Lc = (d1 * d2 * d3_) / (d1 * d2 + d1 * d3_ + d2 * d3_);
   }
-  L[c] = Lc;
-  if constexpr (K == 1) {
-    const double inv_deltat = S->inv_dt;                        // 1.0 / dt
-    const double rn = rho[c];
-    const double nd = mass[c] / V;
-    const double irn = 1.0 / rn, ind = 1.0 / nd;
-    const double tau = 0.5 * (irn + ind);
-    const double itau = 1. / tau;
-    const double du = qdiv(inv_deltat * (ind - irn), tau, itau);
-    double qn = 0.;
-    const double g = ph.gamma;
-    if (du < 0.0) qn = itau * (-0.5 * Lc * cs[c] * du + (g + 1) / 2.0 * Lc * Lc * du * du);
-    double en;
-    if constexpr (CSTS) {
-      double pforward;
-      en = csts_eint(ph, g, ph.eos, ph.pinf, cs_cn1, cs_cn, cs_cdn, cs_con, e[c], nd, mass[c], p[c], q[c], qn,
-                     pforward);
-      pf[c] = pforward + qn;                                    // the forward force's p + q (q: this cycle's)
-    } else {
-      en = energy_update(ph.with_newton != 0, ph.pseudo_centree != 0, ph.eos, g, ph.pinf, ph.threshold, q[c], qn, ind,
-                         irn, nd, p[c], e[c]);
-    }
-    U[c] = V;
-    U[C + c] = V * nd;
-    U[2 * C + c] = V * nd * en;
-    U[3 * C + c] = V * qn;
-    if (fd.pbphi) { fd.pbphi[c] = nd; fd.pbphi[C + c] = en; fd.pbphi[2 * C + c] = qn; }
-  } else {
-    const double cssum[4] = {cs_cn1, cs_cn, cs_cdn, cs_con};
-    lagrange_thermo_env<K, CSTS>(ph, S, env, (int)c, (int)C, V, Lc, rho, e, q, p, cs, mass, U, Vlag, fd.pbphi, cssum,
-                                 pf);
-  }
-  if constexpr (F32) face_data<float>(dm, i, j, k, xr, F3{0.f, 0.f, 0.f}, n0, vh, fd);
-  else face_data<double, HC>(dm, i, j, k, x, xc, n0, vh, fd);
+  const ThermoIn in{V, S->inv_dt, rho[c], mass[c], cs[c], p[c], q[c], e[c]};
+  cell_thermo<K, CSTS, F32>(ph, env, fd, (int)c, (int)C, in, Lc, rho, L, U, Vlag, cs_cn1, cs_cn, cs_cdn, cs_con, pf);
+  auto normal = [&](long long f) { return d3(n0[f], n0[dm.F + f], n0[2 * dm.F + f]); };
+  auto nlo = [&](int d) { return normal(dm.fid(d, i, j, k)); };
+  auto nhi = [&](int d) { return normal(dm.fid(d, i + (d == 0), j + (d == 1), k + (d == 2))); };
+  auto vn = [&](int a) {
+    const long long nn = dm.nid(i + kCellNodeOff[a][0], j + kCellNodeOff[a][1], k + kCellNodeOff[a][2]);
+    return d3(vh[nn], vh[dm.N + nn], vh[2 * dm.N + nn]);
+  };
+  if constexpr (F32) face_data<float, false>(dm, i, j, k, xr, F3{0.f, 0.f, 0.f}, fd, nlo, nhi, vn);
+  else face_data<double, HC>(dm, i, j, k, x, xc, fd, nlo, nhi, vn);
 }
 
 template <int K, typename R, bool HC = false>
@@ -454,6 +525,242 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_cyc_lagrange_ce
                                              env, Vlag, blockIdx.x, linear ? -1 : (int)blockIdx.y, blockIdx.z);
 }
 
+// ------------------------------------------------------------------------
+// The cell kernel over columns of cells (all but schema-csts).  A block takes
+// kColThreads consecutive cells of one z layer (x fastest) and marches up a
+// segment of layers.  The node planes it needs are copied to shared memory one
+// layer ahead (cp.async), so that their latency passes under the arithmetic of
+// the layer before, and each node's Lagrangian coordinates are formed once a
+// block instead of once for each of its 8 cells.  The cell's own state and the
+// normals of its faces are copied at the start of its layer and used at its end.
+// Bound: FP64 latency with 12 warps an SM (168 registers hold the corner
+// vectors' sums; the FP64 pipe is 46 % busy, its work alone takes 150 us and the
+// bytes 165 us on Sedov 128^3).  Measured on B200 against one thread a cell with
+// the nodes gathered from memory: 323 -> 307-315 us there (428 -> 48 bytes of
+// spills), 1372 -> 1156-1233 us on a batch of 24 meshes 32^3..96^3, 868 ->
+// 807-850 us with two gases on 256x128x128.
+constexpr int kColThreads = 128;
+constexpr int kColLayers = 8;        // layers a segment
+constexpr int kColPriv = 24;         // doubles a cell: 18 normals (low and high faces), 6 state values
 
+// Nodes of a strip: a plane of nodes comes as two strips, from the low row of
+// the block's first cell onwards and from one row up; a strip holds the block's
+// cells, one node more a row that it touches and one for its last cell.
+__host__ __device__ __forceinline__ int col_strip(int nx) { return kColThreads + (kColThreads + nx - 2) / nx + 2; }
+__host__ __device__ __forceinline__ size_t col_smem(int nx) {
+  return (size_t)(3 * 12 * col_strip(nx) + kColPriv * kColThreads) * sizeof(double);
+}
+// Blocks of a layer and segments of the column; short columns of small meshes
+// are cut finer so that the blocks fill the chip (3 blocks on 148 SMs).
+__host__ __device__ __forceinline__ int col_blocks(int nx, int ny) { return (nx * ny + kColThreads - 1) / kColThreads; }
+__host__ __device__ __forceinline__ int col_segments(int nx, int ny, int nz) {
+  const int by_len = (nz + kColLayers - 1) / kColLayers, fill = (444 + col_blocks(nx, ny) - 1) / col_blocks(nx, ny);
+  const int want = fill < nz ? fill : nz;
+  return by_len > want ? by_len : want;
+}
+
+__device__ __forceinline__ void cp_async8(double* s, const double* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
+template <int Left> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(Left) : "memory"); }
+
+template <int K, bool HC>
+__device__ __forceinline__ void lagrange_columns(const CycleArgs& A, int bx, int seg) {
+  extern __shared__ double col_mem[];
+  const Dims& dm = A.dm;
+  const int nx = dm.nx, ny = dm.ny, nz = dm.nz, nnx = nx + 1, np = nnx * (ny + 1);
+  const int strip = col_strip(nx), tid = threadIdx.x;
+  const int N = (int)dm.N, C = (int)dm.C, F = (int)dm.F;
+  double* const priv = col_mem + 36 * strip;                      // [kColPriv][kColThreads]
+  const int nseg = col_segments(nx, ny, nz);
+  const int k0 = (int)((long long)nz * seg / nseg), k1 = (int)((long long)nz * (seg + 1) / nseg);
+  const int p0 = bx * kColThreads, p = p0 + tid;
+  const bool cell = p < nx * ny;
+  const int i = p % nx, j = p / nx;
+  const int b0 = p0 + p0 / nx;                                    // plane index of the first cell's node
+  const int off = p + j - b0;                                     // this cell's node (i, j) in the low strip
+  const double dt = A.S->dt, inv_dt = A.S->inv_dt;
+
+  // node plane k -> buffer k % 3: x0 (planes 0..2) and vh (3..5) of both strips
+  auto fetch = [&](int k) {
+    double* buf = col_mem + (k % 3) * 12 * strip;
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      for (int t = tid; t < strip; t += kColThreads) {
+        const int n = b0 + s * nnx + t;
+        if (n < np) {
+          const int g = n + np * k;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            cp_async8(buf + (s * 6 + c) * strip + t, A.x0 + c * N + g);
+            cp_async8(buf + (s * 6 + 3 + c) * strip + t, A.vh + c * N + g);
+          }
+        }
+      }
+  };
+  // the elements this thread copied: coordinates x0 -> x0 + vh dt
+  auto advance = [&](int k) {
+    double* buf = col_mem + (k % 3) * 12 * strip;
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      for (int t = tid; t < strip; t += kColThreads)
+        if (b0 + s * nnx + t < np) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            buf[(s * 6 + c) * strip + t] = buf[(s * 6 + c) * strip + t] + buf[(s * 6 + 3 + c) * strip + t] * dt;
+        }
+  };
+  fetch(k0);
+  fetch(k0 + 1);
+  cp_commit();
+  cp_wait<0>();
+  advance(k0);
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    cp_wait<0>();
+    advance(k + 1);
+    __syncthreads();                       // plane k + 1 is whole; plane k - 1 is read by nobody any more
+    const int c = p + nx * ny * k;
+    if (cell) {
+      // normals: low face of x, y, z, then high; rho, mass, cs, p, q, e
+      const int fx = i + nnx * (j + ny * k), fy = (int)dm.Fx + i + nx * (j + (ny + 1) * k), fz = (int)(dm.Fx + dm.Fy) + c;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double* na = A.n0 + (long long)a * F;
+        cp_async8(priv + (0 + a) * kColThreads + tid, na + fx);
+        cp_async8(priv + (3 + a) * kColThreads + tid, na + fy);
+        cp_async8(priv + (6 + a) * kColThreads + tid, na + fz);
+        cp_async8(priv + (9 + a) * kColThreads + tid, na + fx + 1);
+        cp_async8(priv + (12 + a) * kColThreads + tid, na + fy + nx);
+        cp_async8(priv + (15 + a) * kColThreads + tid, na + fz + nx * ny);
+      }
+      cp_async8(priv + 18 * kColThreads + tid, A.st.rho + c);
+      cp_async8(priv + 19 * kColThreads + tid, A.st.mass + c);
+      cp_async8(priv + 20 * kColThreads + tid, A.st.cs + c);
+      cp_async8(priv + 21 * kColThreads + tid, A.st.p + c);
+      cp_async8(priv + 22 * kColThreads + tid, A.st.q + c);
+      cp_async8(priv + 23 * kColThreads + tid, A.st.e + c);
+    }
+    cp_commit();
+    if (k + 1 < k1) fetch(k + 2);
+    cp_commit();
+    const double* const lo = col_mem + (k % 3) * 12 * strip + off;
+    const double* const hi = col_mem + ((k + 1) % 3) * 12 * strip + off;
+    // component a of the vector at node n of the cell (first = 0: coordinates, 3: velocities)
+    auto node = [&](int n, int first) {
+      const double* b = (n < 4 ? lo : hi) + (kCellNodeOff[n][1] * 6 + first) * strip + kCellNodeOff[n][0];
+      return d3(b[0], b[strip], b[2 * strip]);
+    };
+    if (cell) {
+      double V = 0;
+      {
+        D3 x[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) x[a] = node(a, 0);
+        // corner vectors and volume V = 1/3 sum x_a . cqs_a (MahycoModule.cc:1224-1262)
+        double dvv[8];
+        corner_vectors<double>(x, [&](int a, D3 o) {
+          A.cqs[(a * 3 + 0) * C + c] = o.x; A.cqs[(a * 3 + 1) * C + c] = o.y; A.cqs[(a * 3 + 2) * C + c] = o.z;
+          dvv[a] = dot(x[a], o);
+        });
+#pragma unroll
+        for (int a = 0; a < 8; ++a) V += dvv[a];
+        V *= 1. / 3;
+      }
+      cp_wait<1>();                        // the cell's own state and normals; the next plane may still be on its way
+      // the nodes again from shared memory: holding them through the corner vectors would spill
+      D3 x[8];
+      D3 sm = d3(0., 0., 0.);
+#pragma unroll
+      for (int a = 0; a < 8; ++a) { x[a] = node(a, 0); sm = sm + x[a]; }
+      const D3 xc = .125 * sm;
+      const double* const pv = priv + tid;
+      const ThermoIn in{V, inv_dt, pv[18 * kColThreads], pv[19 * kColThreads], pv[20 * kColThreads],
+                        pv[21 * kColThreads], pv[22 * kColThreads], pv[23 * kColThreads]};
+      auto nlo = [&](int d) { const double* b = pv + 3 * d * kColThreads; return d3(b[0], b[kColThreads], b[2 * kColThreads]); };
+      auto nhi = [&](int d) { const double* b = pv + (9 + 3 * d) * kColThreads; return d3(b[0], b[kColThreads], b[2 * kColThreads]); };
+      auto vn = [&](int a) { return node(a, 3); };
+      double Lc = 0.;
+      A.xc[c] = xc.x; A.xc[C + c] = xc.y; A.xc[2 * C + c] = xc.z;
+      if (A.ph.lc_mode != 0) Lc = face_length(x);
+      cell_thermo<K, false, false>(A.ph, A.env, A.fd, c, C, in, Lc, A.st.rho, A.L, A.U[0], A.Vlag, 0., 0., 0., 0., nullptr);
+      face_data<double, HC>(dm, i, j, k, x, xc, A.fd, nlo, nhi, vn);
+    }
+  }
+}
+
+template <int K, bool HC = false>
+__global__ void __launch_bounds__(kColThreads, 3) k_cyc_lagrange_columns(const __grid_constant__ CycleArgs a) {
+  lagrange_columns<K, HC>(a, blockIdx.x, blockIdx.y);
+}
+
+// The same over a batch's column table (instance, chunk, segment).  The
+// instance's arguments are read from shared memory where they are used:
+// fifty pointers in registers would spill.
+template <int K, bool HC = false>
+__global__ void __launch_bounds__(kColThreads, 3) k_bat_lagrange_columns(const CycleArgs* __restrict__ D,
+                                                                         const int4* __restrict__ W, int nw) {
+  __shared__ CycleArgs a;
+  for (int w = blockIdx.x; w < nw; w += gridDim.x) {
+    const int4 t = W[w];
+    __syncthreads();                       // the previous item's reads are done
+    static_assert(sizeof(CycleArgs) % sizeof(double) == 0, "copied as doubles");
+    for (int x = threadIdx.x; x < (int)(sizeof(CycleArgs) / sizeof(double)); x += kColThreads)
+      reinterpret_cast<double*>(&a)[x] = reinterpret_cast<const double*>(D + t.x)[x];
+    __syncthreads();
+    lagrange_columns<K, HC>(a, t.y, t.z);
+  }
+}
+
+// Whether a context's FP64 cell kernel takes columns: not on small meshes, whose
+// few blocks do not hide the copy of the first planes (100x5x5: 13.9 us against
+// 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1).
+constexpr long long kColMinCells = 65536;
+
+template <class Kern>
+static void launch_columns(Kern kern, const CycleArgs& a, cudaStream_t s) {
+  const Dims& dm = a.dm;
+  const size_t smem = col_smem(dm.nx);
+  smem_opt_in((const void*)kern, smem);
+  kern<<<dim3(col_blocks(dm.nx, dm.ny), col_segments(dm.nx, dm.ny, dm.nz)), kColThreads, smem, s>>>(a);
+}
+// The cell kernel of a context, all but schema-csts.
+template <int K>
+static void launch_cells(const CycleArgs& a, cudaStream_t s) {
+  const bool hc = a.fd.h != nullptr;               // cell widths: order 3 or the generalised limiters
+  if (!a.ph.precision && a.dm.C >= kColMinCells) {
+    if (hc) launch_columns(k_cyc_lagrange_columns<K, true>, a, s);
+    else launch_columns(k_cyc_lagrange_columns<K, false>, a, s);
+    return;
+  }
+  int linear;
+  const dim3 nbc = cell_grid(a.dm, linear);
+  auto kern = a.ph.precision ? k_cyc_lagrange_cells<K, float> : (hc ? k_cyc_lagrange_cells<K, double, true> : k_cyc_lagrange_cells<K, double>);
+  kern<<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p, a.st.cs, a.st.mass,
+                           a.cqs, a.cqs32, a.L, a.U[0], a.xc, a.fd, a.env, a.Vlag, linear);
+}
+
+template <class Kern>
+static void launch_bat_columns(Kern kern, const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  smem_opt_in((const void*)kern, P.col_smem);
+  if (P.ncwork > 0)
+    kern<<<persistent_grid((const void*)kern, kColThreads, P.col_smem, P.ncwork, P.occ_pct[BK_LCELLS]), kColThreads,
+           P.col_smem, s>>>(P.descs, P.cwork, P.ncwork);
+  mark(m, BK_LCELLS, s);
+}
+
+// A batch's mixed form and schema-csts: the cell tiles of BK_LCELLS.
+template <int K, typename R, bool HC, bool CSTS>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_lagrange_cells(const CycleArgs* __restrict__ D,
+                                                                                   const int4* __restrict__ W, int nw) {
+  for (int w = blockIdx.x; w < nw; w += gridDim.x) {
+    const int4 t = W[w];
+    const CycleArgs& a = D[t.x];
+    k_cyc_lagrange_cells_body<K, R, CSTS, HC>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p,
+                                              a.st.cs, a.st.mass, a.cqs, CSTS ? nullptr : a.cqs32, a.L, a.U[0], a.xc,
+                                              a.fd, a.env, a.Vlag, t.y, t.z, t.w, a.vnb, a.pf);
+  }
+}
 
 }  // namespace mhy

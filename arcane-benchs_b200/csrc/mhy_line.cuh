@@ -72,7 +72,7 @@ __device__ __forceinline__ void finalize_cell(const Phys& ph, const Scalars* S, 
   double fvol = U0 * unsurvolt;
   if (fvol < thr) fvol = 0.;
   const double somme_frac = 0. + fvol;
-  const double unsursomme_frac = 1. / somme_frac;
+  const double unsursomme_frac = rc<double, SP>(somme_frac, oor);
   fvol = fvol * unsursomme_frac;
   double mf = 1., unsurmasset = 0.;
   if (masset != 0.) {
@@ -80,7 +80,7 @@ __device__ __forceinline__ void finalize_cell(const Phys& ph, const Scalars* S, 
     mf = U1 * unsurmasset;
     if (fvol < thr) mf = 0.;
     const double fmasset = 0. + mf;
-    if (fmasset != 0.) { const double unsurfmasset = 1. / fmasset; mf = mf * unsurfmasset; }
+    if (fmasset != 0.) { const double unsurfmasset = rc<double, SP>(fmasset, oor); mf = mf * unsurfmasset; }
   } else {
     atomicOr(&const_cast<Scalars*>(S)->status, MHY_STATUS_ZERO_MASS);
   }
@@ -158,20 +158,14 @@ __device__ __forceinline__ void face_grad(bool inner, R dx, const R Pn[4], const
   if constexpr (SP) { if ((threadIdx.x & 31) != 0) *oor |= fo; }
 }
 
-// Limited cell gradient from the back and front face gradients (R:497-506).
-template <typename R, bool SP = false>
-__device__ __forceinline__ R limited_one(int lim, R gb, R gf, unsigned* oor = nullptr) {
-  return limited_slope<R, false, SP>(lim, gb, gf, oor);
-}
-
+// Limited cell gradients from the back and front face gradients (R:497-506).
 // Variable 0 (the volume) has Phi = U0/U0 = 1 on every cell of a
 // single-environment mesh, so its face gradients are zero and its limited
 // gradient is +0; only variables 1..3 are computed.
 template <typename R, bool SP = false>
 __device__ __forceinline__ void limited_grad(int lim, const R gb[4], const R gf[4], R G[4], unsigned* oor = nullptr) {
   G[0] = 0;
-#pragma unroll
-  for (int v = 1; v < 4; ++v) G[v] = limited_one<R, SP>(lim, gb[v], gf[v], oor);
+  limited_slopes<3, R, false, SP>(lim, gb + 1, gf + 1, G + 1, oor);
 }
 
 // Upwind face value (R:707-714): from the previous cell when u_f dx_f > 0.
@@ -406,7 +400,7 @@ __device__ __forceinline__ void cell_line(const Phys& ph, double dt, const Scala
     for (int v = 0; v < 4; ++v) { Pne[v] = infr ? Pn[v] : P[v]; Ppe[v] = inner ? Pp[v] : P[v]; }
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      G[v] = lim < 3 ? limited_one<R>(lim, g[v], gr[v])
+      G[v] = lim < 3 ? limited_slope<R, false>(lim, g[v], gr[v])
                      : flux_limiter_g<R>(lim, gr[v], g[v], P[v], Pne[v], Ppe[v], h0, hp, hm);
     const double un = __shfl_down_sync(full, in.u, 1);
     const double ob = in.ob * in.u, of = in.of * un;                 // outward velocities of the two faces
@@ -604,8 +598,7 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
       }
     } else if (valid && inner) {
       unsigned go = 0u;                               // lanes 1..30: what reaches an updated node
-#pragma unroll
-      for (int c = 0; c < 3; ++c) G[c] = limited_slope<R, true, SP>(lim, gb[c], gf[c], &go);
+      limited_slopes<3, R, true, SP>(lim, gb, gf, G, &go);
       if constexpr (SP) { const int lane = threadIdx.x & 31; if (lane >= 1 && lane <= 30) *oor |= go; }
     }
   }
@@ -1019,9 +1012,6 @@ __global__ void __launch_bounds__(32 * W, TileGeom<W>::minb) k_cyc_sweep_nodes_t
 
 // ------------------------------------------------------------------------
 // Host-side node sweep launchers.
-
-// Dynamic shared memory above the default 48 KB needs an opt-in per kernel and device.
-void smem_opt_in(const void* kernel, size_t bytes);
 
 template <int D, bool FIRST, bool LAST, int K, typename R, int W, bool GL = false>
 static void sweep_nodes_launch_w(const CycleArgs& a, int prev, const double* udin, double* udout, cudaStream_t s) {

@@ -63,8 +63,8 @@ __device__ __forceinline__ void face_values_env(const Phys& ph, int lim, bool in
                xpz = __shfl_up_sync(full, in.xc[2], 1);
   const double dx = inner ? dot(d3(in.xc[0], in.xc[1], in.xc[2]) - d3(xpx, xpy, xpz), d3(in.n[0], in.n[1], in.n[2]))
                           : 0.;
-  unsigned fo = 0u, go = 0u;
-  const R dxR = (R)dx, rdx = inner ? rc<R, SP>(dxR, &fo) : R(0);
+  unsigned fo = 0u;
+  const R dxR = (R)dx, rdx = inner ? R(1) / dxR : R(0);
   R G[NV], Pp[NV];
   R h0 = R(0), hm = R(0), hp = R(0);
   if constexpr (GL) {
@@ -78,19 +78,14 @@ __device__ __forceinline__ void face_values_env(const Phys& ph, int lim, bool in
     const R gr = __shfl_down_sync(full, g, 1);
     if constexpr (GL) {
       const R Pn = __shfl_down_sync(full, P[v], 1);
-      G[v] = lim < 3 ? limited_one<R>(lim, g, gr)
+      G[v] = lim < 3 ? limited_slope<R, false>(lim, g, gr)
                      : flux_limiter_g<R>(lim, gr, g, P[v], infr ? Pn : P[v], inner ? Pp[v] : P[v], h0, hp, hm);
     } else {
-      G[v] = limited_one<R, SP>(lim, g, gr, &go);
+      G[v] = limited_slope<R, false>(lim, g, gr);
     }
   }
-  // lane 0's back neighbour is itself (0 / 0): its face gradient reaches no
-  // updated cell, and only the limited gradients of lanes 1..30 do
-  if constexpr (SP) {
-    const int lane = threadIdx.x & 31;
-    if (lane != 0) *oor |= fo;
-    if (lane >= 1 && lane <= 30) *oor |= go;
-  }
+  // lane 0's back neighbour is itself (0 / 0): its gradient reaches no updated cell
+  if constexpr (SP) { if ((threadIdx.x & 31) != 0) *oor |= fo; }
   const bool back = in.u * dx > 0.0;
   const R dot_xf = (R)(back ? in.db : in.df);
 #pragma unroll
@@ -207,7 +202,7 @@ __device__ __forceinline__ void cell_line_env(const Phys& ph, double dt, bool va
 #pragma unroll
           for (int k = 0; k < K; ++k) den += in.U[k];
         }
-        const R dR = (R)den, r = rc<R, SP>(dR, oor);
+        const R dR = (R)den, r = R(1) / dR;
 #pragma unroll
         for (int v = 0; v < NV; ++v) P[v] = dv<R, SP>((R)in.U[v], dR, r, oor);
       }
@@ -236,7 +231,7 @@ __device__ __forceinline__ void cell_line_env(const Phys& ph, double dt, bool va
         Pne[v] = infr ? Pn : P[v]; Ppe[v] = inner ? Pp : P[v];
         const double g = inner ? qdiv(P[v] - Pp, dx, rdx) : 0.;
         const double gr = __shfl_down_sync(full, g, 1);
-        G[v] = lim < 3 ? limited_one<double>(lim, g, gr)
+        G[v] = lim < 3 ? limited_slope<double, false>(lim, g, gr)
                        : flux_limiter_g<double>(lim, gr, g, P[v], Pne[v], Ppe[v], h0, hp, hm);
       }
       const double un = __shfl_down_sync(full, in.u, 1);
@@ -1043,28 +1038,11 @@ static void set_env_attributes() {
   set_env_attributes_r<K, float>();
 }
 
-template <int K, typename R>
-static void lagrange_cells_env(const CycleArgs& a, const dim3 nbc, int linear, cudaStream_t s) {
-  auto kern = k_cyc_lagrange_cells<K, R>;
-  if constexpr (sizeof(R) == 8)
-    if (a.fd.h) kern = k_cyc_lagrange_cells<K, R, true>;   // cell widths: order 3 and the generalised limiters
-  kern<<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p, a.st.cs, a.st.mass,
-                           a.cqs, a.cqs32, a.L, a.U[0], a.xc, a.fd, a.env, a.Vlag, linear);
-}
-
 void launch_lagrange_cells_env(const CycleArgs& a, cudaStream_t s) {
   if (a.ph.csts) { launch_lagrange_cells_csts_env(a, s); return; }
-  int linear;
-  const dim3 nbc = cell_grid(a.dm, linear);
-  if (a.ph.precision) {
-    if (a.K == 2) lagrange_cells_env<2, float>(a, nbc, linear, s);
-    else if (a.K == 3) lagrange_cells_env<3, float>(a, nbc, linear, s);
-    else lagrange_cells_env<4, float>(a, nbc, linear, s);
-  } else {
-    if (a.K == 2) lagrange_cells_env<2, double>(a, nbc, linear, s);
-    else if (a.K == 3) lagrange_cells_env<3, double>(a, nbc, linear, s);
-    else lagrange_cells_env<4, double>(a, nbc, linear, s);
-  }
+  if (a.K == 2) launch_cells<2>(a, s);
+  else if (a.K == 3) launch_cells<3>(a, s);
+  else launch_cells<4>(a, s);
 }
 
 void launch_remap_env(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m) {
@@ -1088,18 +1066,6 @@ void launch_remap_env(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks
 // single-context kernels, driven by the batch's work tables over persistent
 // grids (as the one-environment batch in mhy_cycle.cu).  The cell y/z sweeps
 // take 8 or 16 lines per block, the node y/z sweeps 8, as in one context.
-
-template <int K, typename R, bool HC, bool CSTS = false>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_env_lagrange_cells(
-    const CycleArgs* __restrict__ D, const int4* __restrict__ W, int nw) {
-  for (int w = blockIdx.x; w < nw; w += gridDim.x) {
-    const int4 t = W[w];
-    const CycleArgs& a = D[t.x];
-    k_cyc_lagrange_cells_body<K, R, CSTS, HC>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p,
-                                              a.st.cs, a.st.mass, a.cqs, CSTS ? nullptr : a.cqs32, a.L, a.U[0], a.xc,
-                                              a.fd, a.env, a.Vlag, t.y, t.z, t.w, a.vnb, a.pf);
-  }
-}
 
 template <int K, bool FIRST, typename R, bool GL, bool PB = false, bool O3 = false>
 __global__ void __launch_bounds__(32 * kLineWarps, kEnvMinBlocks) k_bat_env_cells_x(
@@ -1267,15 +1233,17 @@ static void batch_cycle_env(const BatchPlan& P, int sens, cudaStream_t s, Kernel
   bool done = false;
   if constexpr (sizeof(R) == 8) {
     if (P.csts) {   // schema-csts: the cell kernel's CSTS form, then the forward step and the face velocities
-      bat_env_launch(k_bat_env_lagrange_cells<K, R, HC, true>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
+      bat_env_launch(k_bat_lagrange_cells<K, double, HC, true>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
                      P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
       launch_bat_csts_forward(P, s);
       done = true;
     }
   }
-  if (!done)
-    bat_env_launch(k_bat_env_lagrange_cells<K, R, HC>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
-                   P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+  if (!done) {
+    if constexpr (sizeof(R) == 8) launch_bat_columns(k_bat_lagrange_columns<K, HC>, P, s, m);
+    else bat_env_launch(k_bat_lagrange_cells<K, float, false, false>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
+                        P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+  }
   int prev = 0;
   for (int it = 0; it < 3; ++it) {
     const int d = (it + sens) % 3;

@@ -60,23 +60,12 @@ MHY_POW_HD double pow3_fma(double a, double b, double c) {
 #endif
 }
 
-// V^(1./3.) for V > 0; NaN for V < 0 or NaN, 0 for +-0, +inf for +inf (the
-// values std::pow returns for these arguments with a positive non-integer exponent).
-MHY_POW_HD double pow_third(double v) {
-  if (!(v > 0.0)) {
-    if (v == 0.0) return 0.0;
-    return pow3_from_bits(0x7ff8000000000000ull);      // NaN
-  }
-  uint64_t b = pow3_bits(v);
-  int be = (int)((b >> 52) & 0x7ff);
-  if (be == 0x7ff) return v;                            // +inf
-  int ex_adj = 0;
-  if (be == 0) {                                        // subnormal: scale by 2^120 (exact)
-    v = v * pow3_from_bits((uint64_t)(1023 + 120) << 52);
-    b = pow3_bits(v);
-    be = (int)((b >> 52) & 0x7ff);
-    ex_adj = -120;
-  }
+// V^(1./3.) of a normal V > 0 scaled by 2^-ex_adj beforehand; quo(x, y) is the
+// correctly rounded x / y.
+template <typename Quo>
+MHY_POW_HD double pow_third_normal(double v, int ex_adj, Quo&& quo) {
+  const uint64_t b = pow3_bits(v);
+  const int be = (int)((b >> 52) & 0x7ff);
   const int ex = be - 1023 + ex_adj;                    // V = m * 2^ex, m in [1,2)
   const double m = pow3_from_bits((b & 0x000fffffffffffffull) | (0x3ffull << 52));
 
@@ -115,7 +104,7 @@ MHY_POW_HD double pow_third(double v) {
   double mm = m;
   int exl = ex;
   if (mm > 1.4142135623730951) { mm = mm * 0.5; exl += 1; }
-  const double s = (mm - 1.0) / (mm + 1.0);
+  const double s = quo(mm - 1.0, mm + 1.0);
   const double s2 = s * s;
   // 2*(s + s^3/3 + ... + s^15/15): truncation < 1e-13 for |s| <= 0.1716
   double poly = 1.0 / 15.0;
@@ -137,6 +126,23 @@ MHY_POW_HD double pow_third(double v) {
   const int q1 = q / 2, q2 = q - q1;
   return out * pow3_from_bits((uint64_t)(1023 + q1) << 52)
              * pow3_from_bits((uint64_t)(1023 + q2) << 52);
+}
+
+// V^(1./3.) for V > 0; NaN for V < 0 or NaN, 0 for +-0, +inf for +inf (the
+// values std::pow returns for these arguments with a positive non-integer exponent).
+MHY_POW_HD double pow_third(double v) {
+  if (!(v > 0.0)) {
+    if (v == 0.0) return 0.0;
+    return pow3_from_bits(0x7ff8000000000000ull);      // NaN
+  }
+  const int be = (int)((pow3_bits(v) >> 52) & 0x7ff);
+  if (be == 0x7ff) return v;                            // +inf
+  int ex_adj = 0;
+  if (be == 0) {                                        // subnormal: scale by 2^120 (exact)
+    v = v * pow3_from_bits((uint64_t)(1023 + 120) << 52);
+    ex_adj = -120;
+  }
+  return pow_third_normal(v, ex_adj, [](double x, double y) { return x / y; });
 }
 
 }  // namespace mhy

@@ -76,8 +76,9 @@ MHY_Q_HD double rcp_from_seed(double y, double y0, unsigned& bad) {
   const double y1 = q_fma(y0, q_fma(d, d, d), y0);
   const double r = q_fma(y1, q_fma(-y, y1, 1.0), y1);
   const uint32_t h = q_hi(y);
-  if (MHY_Q_OUT(h, 64, 1983) || (q_lo(y) & (h | 0xfff00000u)) == 0xffffffffu) bad = 1u;
-  return r;
+  if (MHY_Q_OUT(h, 64, 1983)) bad = 1u;
+  const uint32_t ones = (q_lo(y) & (h | 0xfff00000u)) == 0xffffffffu ? 1u : 0u;
+  return q_make(q_hi(r), q_lo(r) | ones);
 }
 
 // RN(x/y) with r = RN(1/y); a zero x gives the zero of the right sign (q0's).

@@ -77,12 +77,12 @@ def lib(tmp_path_factory):
 def test_unflagged_results_are_ieee_division(lib, span, seed_error):
     flagged = ctypes.c_long()
     assert lib.check(2_000_000, 17 + span, span, seed_error, ctypes.byref(flagged)) == 0
-    assert flagged.value < 0.03 * 2_000_000       # only all-ones significands of y, and few quotients out of range
+    assert flagged.value < 0.03 * 2_000_000       # few quotients out of range
 
 
 @pytest.mark.parametrize("x,y,expected", [
     (1.0, 3.0, 0), (0.0, 3.0, 0), (-0.0, 3.0, 0), (1.0, 0.0, 1), (0.0, 0.0, 1), (1.0, float("inf"), 1),
     (float("nan"), 1.0, 1), (1.0, float("nan"), 1), (float("inf"), 1.0, 1), (1e-300, 1.0, 1), (5e-324, 1.0, 1),
-    (1.0, 1e-300, 1), (1e-200, 1e200, 1), (1e250, 1e-250, 1), (1.0, 1.0 - 2.0 ** -53, 1), (1e-280, 1e-280, 0)])
+    (1.0, 1e-300, 1), (1e-200, 1e200, 1), (1e250, 1e-250, 1), (1.0, 1.0 - 2.0 ** -53, 0), (1e-280, 1e-280, 0)])
 def test_flag(lib, x, y, expected):
     assert (lib.flag(x, y) != 0) == bool(expected)
