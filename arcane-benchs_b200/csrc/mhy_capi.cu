@@ -707,6 +707,7 @@ struct mhy_batch {
   std::vector<mhy_ctx*> inst;
   CycleArgs* d_descs = nullptr;
   int4* d_work[BK_COUNT] = {};
+  int4* d_mwork[BK_COUNT] = {};                 // marching sweeps
   int4* d_cwork = nullptr;                      // the Lagrange cell kernel's columns
   int4* d_o3work[3] = {};                       // order 3: face work tables per direction
   int4* d_fwork = nullptr;                      // schema-csts: face work table (all directions)
@@ -725,7 +726,7 @@ namespace {
 // one of three orders (mhy_tuning.order), for the given lines per block.
 // kColumns instead of a kind: the columns of the Lagrange cell kernel.
 constexpr int kColumns = -1;
-std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int order, int lines) {
+std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int order, int lines, bool march) {
   const int n = (int)inst.size();
   std::vector<int> ids(n);
   std::iota(ids.begin(), ids.end(), 0);
@@ -739,7 +740,7 @@ std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int or
       batch_column_shape(inst[i]->dm, gx, gy, smem);
       gz = 1;
     } else {
-      batch_work_shape(inst[i]->dm, kind, lines, gx, gy, gz);
+      batch_work_shape(inst[i]->dm, kind, lines, march, gx, gy, gz);
     }
     if (gy < 0) {                               // linear chunks of consecutive items
       for (int x = 0; x < gx; ++x) per[i].push_back(make_int4(i, x, -1, 0));
@@ -774,6 +775,7 @@ void mhy_batch_destroy(mhy_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (int s = 0; s < 3; ++s) if (b->graph[s]) cudaGraphExecDestroy(b->graph[s]);
   for (int k = 0; k < BK_COUNT; ++k) if (b->d_work[k]) cudaFree(b->d_work[k]);
+  for (int k = 0; k < BK_COUNT; ++k) if (b->d_mwork[k]) cudaFree(b->d_mwork[k]);
   if (b->d_cwork) cudaFree(b->d_cwork);
   for (int d = 0; d < 3; ++d) if (b->d_o3work[d]) cudaFree(b->d_o3work[d]);
   if (b->d_fwork) cudaFree(b->d_fwork);
@@ -809,20 +811,32 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
   b->device = b->inst[0]->device;
   cudaError_t err = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_CUDA, cudaGetErrorString(err)); }
+  long long nodes = 0;
+  for (const mhy_ctx* c : b->inst) nodes += c->dm.N;
   // work tables: every block of every instance's grid, instance-major
   for (int k = 0; k < BK_COUNT; ++k) {
     // capacity for the largest table any tuning builds (8 lines per block)
     size_t cap = 0;
-    for (int lw : kLineOptions) cap = std::max(cap, build_work(b->inst, k, 0, lw).size());
-    const std::vector<int4> w = build_work(b->inst, k, 0, kLineWarps);
+    for (int lw : kLineOptions) cap = std::max(cap, build_work(b->inst, k, 0, lw, false).size());
+    const std::vector<int4> w = build_work(b->inst, k, 0, kLineWarps, false);
     err = cudaMalloc(&b->d_work[k], cap * sizeof(int4));
     if (err == cudaSuccess) err = cudaMemcpy(b->d_work[k], w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
     b->plan.work[k] = b->d_work[k];
     b->plan.nwork[k] = (int)w.size();
+    b->plan.march[k] = batch_marches(b->inst[0]->args(), k, nodes);
+    if (!b->plan.march[k]) continue;
+    cap = 0;
+    for (int lw : kLineOptions) cap = std::max(cap, build_work(b->inst, k, 0, lw, true).size());
+    const std::vector<int4> mw = build_work(b->inst, k, 0, kLineWarps, true);
+    err = cudaMalloc(&b->d_mwork[k], cap * sizeof(int4));
+    if (err == cudaSuccess) err = cudaMemcpy(b->d_mwork[k], mw.data(), mw.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
+    b->plan.mwork[k] = b->d_mwork[k];
+    b->plan.nmwork[k] = (int)mw.size();
   }
   {
-    const std::vector<int4> w = build_work(b->inst, kColumns, 0, kLineWarps);
+    const std::vector<int4> w = build_work(b->inst, kColumns, 0, kLineWarps, false);
     err = cudaMalloc(&b->d_cwork, w.size() * sizeof(int4));
     if (err == cudaSuccess) err = cudaMemcpy(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
@@ -1021,15 +1035,21 @@ int check_tuning(const mhy_tuning& t) {
 int apply_tuning(mhy_batch* b, const mhy_tuning& t) {
   for (int k = 0; k < BK_COUNT; ++k) {
     if (t.order[k] == b->order[k] && t.lines_per_block[k] == b->plan.lines[k]) continue;
-    const std::vector<int4> w = build_work(b->inst, k, t.order[k], t.lines_per_block[k]);
+    const std::vector<int4> w = build_work(b->inst, k, t.order[k], t.lines_per_block[k], false);
     MHY_CUDA(cudaMemcpyAsync(b->d_work[k], w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
     MHY_CUDA(cudaStreamSynchronize(b->stream));                 // w is a host temporary
+    if (b->plan.march[k]) {
+      const std::vector<int4> mw = build_work(b->inst, k, t.order[k], t.lines_per_block[k], true);
+      MHY_CUDA(cudaMemcpyAsync(b->d_mwork[k], mw.data(), mw.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
+      MHY_CUDA(cudaStreamSynchronize(b->stream));
+      b->plan.nmwork[k] = (int)mw.size();
+    }
     b->order[k] = t.order[k];
     b->plan.lines[k] = t.lines_per_block[k];
     b->plan.nwork[k] = (int)w.size();
   }
   if (t.order[BK_LCELLS] != b->col_order) {
-    const std::vector<int4> w = build_work(b->inst, kColumns, t.order[BK_LCELLS], kLineWarps);
+    const std::vector<int4> w = build_work(b->inst, kColumns, t.order[BK_LCELLS], kLineWarps, false);
     MHY_CUDA(cudaMemcpyAsync(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
     MHY_CUDA(cudaStreamSynchronize(b->stream));
     b->col_order = t.order[BK_LCELLS];

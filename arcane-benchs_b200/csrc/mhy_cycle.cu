@@ -20,6 +20,7 @@
 
 #include "mhy_lagrange.cuh"
 #include "mhy_line.cuh"
+#include "mhy_march.cuh"
 
 namespace mhy {
 
@@ -443,6 +444,9 @@ static void sweep_cells_t(const CycleArgs& a, const double* Uin, double* Uout, c
     if (o3) { sweep_cells_t_w<D, LAST, R, kLineWarps, true, false>(a, Uin, Uout, s); return; }
     if (gl) { sweep_cells_t_w<D, LAST, R, kLineWarps, false, true>(a, Uin, Uout, s); return; }
   }
+  if constexpr (sizeof(R) == 4) {
+    if (march_cells(a.dm.N, 1)) { sweep_cells_launch_m<D, LAST>(a, LAST ? 2 : (Uin == a.U[0] ? 0 : 1), s); return; }
+  }
   const int w = a.lines[BK_CELLS_X + D];
   if (w == 32) sweep_cells_t_w<D, LAST, R, 32>(a, Uin, Uout, s);
   else if (w == 16) sweep_cells_t_w<D, LAST, R, 16>(a, Uin, Uout, s);
@@ -680,10 +684,17 @@ void launch_delta_t(const CycleArgs& a, cudaStream_t s) {
 // work item with a barrier, since the previous item's last reads of the tile
 // may still be in flight in other warps.
 
-void batch_work_shape(const Dims& dm, int kind, int lines, int& gx, int& gy, int& gz) {
+void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, int& gy, int& gz) {
   const int nx = dm.nx, ny = dm.ny, nz = dm.nz;
   auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
   const int W = lines;                            // lines per block of the y/z sweeps
+  if (march) {                                    // y/z sweep: chunks of the plane x segments of the lines
+    const bool nodes = kind >= BK_NODES_X;
+    const int D = kind - (nodes ? BK_NODES_X : BK_CELLS_X), e = nodes ? 1 : 0;
+    const int points = (nx + e) * ((D == 1 ? nz : ny) + e);
+    gx = cdiv(points, kMarchThreads); gy = march_segments(dm.ncd(D) + e, points, march_len(lines)); gz = 1;
+    return;
+  }
   switch (kind) {
     case BK_LNODES: gx = (int)cdiv((int)dm.N, 128); gy = -1; gz = 1; break;      // linear chunks
     case BK_LCELLS:
@@ -877,6 +888,14 @@ void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem
   smem = col_smem(dm.nx);
 }
 
+// The y/z sweeps of a batch with a table of marching work (FP64 node sweeps
+// march on the first sweep of a remap only).
+bool batch_marches(const CycleArgs& a, int kind, long long nodes) {
+  if (kind == BK_NODES_Y || kind == BK_NODES_Z) return march_nodes(nodes, a.ph.precision, true);
+  if (kind == BK_CELLS_Y || kind == BK_CELLS_Z) return a.K == 1 && march_cells(nodes, a.ph.precision);
+  return false;
+}
+
 void mark(KernelMarks* m, int kind, cudaStream_t s) {
   if (!m || m->n >= KernelMarks::kMax) return;
   cudaEventRecord(m->ev[m->n], s);
@@ -936,6 +955,13 @@ static void bat_cells_d(const BatchPlan& P, int it, cudaStream_t s, KernelMarks*
     launch_persistent(k_bat_sweep_cells_x<LAST, R, GL>, 32 * kLineWarps, 0, P, kind, kind, s, m, P.descs, P.work[kind],
                       P.nwork[kind], it);
   } else {
+    if constexpr (sizeof(R) == 4) {
+      if (P.march[kind]) {
+        launch_march(k_bat_sweep_cells_m<DD, LAST>, P, kind, s, m, P.descs, P.mwork[kind], P.nmwork[kind], it,
+                     march_len(P.lines[kind]));
+        return;
+      }
+    }
     const int w = P.lines[kind];
     if (GL || w == 8) bat_cells_t<DD, LAST, R, 8, GL>(P, it, s, m);   // the G limiters keep 8 lines
     else if (w == 32) bat_cells_t<DD, LAST, R, 32, false>(P, it, s, m);
@@ -957,6 +983,13 @@ static void bat_nodes_d(const BatchPlan& P, int it, int prev, cudaStream_t s, Ke
     launch_persistent(k_bat_sweep_nodes_x<FIRST, LAST, R, GL>, 32 * kLineWarps, 0, P, kind, kind, s, m, P.descs,
                       P.work[kind], P.nwork[kind], it, prev);
   } else {
+    if constexpr (sizeof(R) == 4 || FIRST) {
+      if (P.march[kind]) {
+        launch_march(k_bat_sweep_nodes_m<DD, FIRST, LAST, 1, R, GL>, P, kind, s, m, P.descs, P.mwork[kind],
+                     P.nmwork[kind], prev, march_len(P.lines[kind]));
+        return;
+      }
+    }
     const int w = P.lines[kind];
     if (GL || w == 8) bat_nodes_t<DD, FIRST, LAST, R, 8, GL>(P, it, prev, s, m);
     else if (w == 32) bat_nodes_t<DD, FIRST, LAST, R, 32, false>(P, it, prev, s, m);

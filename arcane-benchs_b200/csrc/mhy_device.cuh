@@ -168,16 +168,19 @@ __device__ __forceinline__ R limited_slope(int lim, R gb, R gf) {
 // NV of them.  The speculative form takes zero where a pair has opposite signs
 // or a zero.  For superBee and vanLeer it also raises *oor for differences of
 // 1e150 and more, infinities and NaN, whose terms may be other than zero at
-// opposite signs.  Nothing is skipped where there is nothing to limit, so that
-// the slopes overlap.
-template <int NV, typename R, bool DUAL, bool SP>
+// opposite signs.  What it skips where there is nothing to limit (quiescent
+// regions): nothing by default, so that the slopes overlap (the warp-wide line
+// sweeps, many warps in flight); SKIP the set, if all of them are zero (the
+// marching sweeps, few warps: 107 -> 98 us for a node sweep of Sedov 128^3).
+template <int NV, typename R, bool DUAL, bool SP, bool SKIP = false>
 __device__ __forceinline__ void limited_slopes(int lim, const R* gb, const R* gf, R* G, unsigned* oor) {
   const R h = R(0.5), one = R(1), zero = R(0);
   if constexpr (sizeof(R) == 8 && SP) {
-    bool live[NV];
+    bool live[NV], any = false;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       live[v] = !((gb[v] <= zero && gf[v] >= zero) || (gb[v] >= zero && gf[v] <= zero));
+      any = any || live[v];
       G[v] = zero;
     }
     if (lim != 0) {
@@ -185,7 +188,7 @@ __device__ __forceinline__ void limited_slopes(int lim, const R* gb, const R* gf
       for (int v = 0; v < NV; ++v)
         if (!(fabs(gb[v]) < 1e150 && fabs(gf[v]) < 1e150)) *oor = 1u;
     }
-    if (lim >= 0) {                                          // lim < 0: order 1
+    if (lim >= 0 && (any || !SKIP)) {                        // lim < 0: order 1
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         unsigned bad = 0u;

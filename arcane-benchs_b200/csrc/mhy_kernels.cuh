@@ -156,6 +156,9 @@ struct BatchPlan {
   int occ_pct[BK_TUNE_SLOTS];   // persistent grid of each slot: % of the resident-block capacity
   int lines[BK_COUNT];          // lines per block of the y/z sweeps (8, 16, 32); the work shapes follow it
   int K;                        // environments of every instance
+  bool march[BK_COUNT];         // the y/z sweeps that march along lines (the same in every instance),
+  const int4* mwork[BK_COUNT];  // and their work tables (instance, plane chunk, segment)
+  int nmwork[BK_COUNT];
   int gl;                       // every instance takes the G limiters (FP64): the GL sweeps and cell widths
   int pb;                       // every instance takes projection-pente-borne (FP64): the PB cell sweeps
   int o3;                       // every instance takes order 3 (FP64): face values, then the O3 cell sweeps
@@ -177,7 +180,9 @@ struct KernelMarks {
   int kind[kMax];
   int n;
 };
-void batch_work_shape(const Dims& dm, int kind, int lines, int& gx, int& gy, int& gz);
+// Blocks of one instance's grid for a kernel kind; march: its y/z sweep marches (BatchPlan::march).
+void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, int& gy, int& gz);
+bool batch_marches(const CycleArgs& a, int kind, long long nodes);
 void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem);
 // Dynamic shared memory above the default 48 KB needs an opt-in per kernel and device.
 void smem_opt_in(const void* kernel, size_t bytes);

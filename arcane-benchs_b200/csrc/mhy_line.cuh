@@ -1010,65 +1010,4 @@ __global__ void __launch_bounds__(32 * W, TileGeom<W>::minb) k_cyc_sweep_nodes_t
   k_cyc_sweep_nodes_t_body<D, FIRST, LAST, K, R, W, GL>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, udout, dpf, Gd, mass, vout, nm_out, vnorm, blockIdx.x, blockIdx.y, blockIdx.z, ecn);
 }
 
-// ------------------------------------------------------------------------
-// Host-side node sweep launchers.
-
-template <int D, bool FIRST, bool LAST, int K, typename R, int W, bool GL = false>
-static void sweep_nodes_launch_w(const CycleArgs& a, int prev, const double* udin, double* udout, cudaStream_t s) {
-  const Dims& dm = a.dm;
-  const int nseg = (dm.ncd(D) + 1 + kLineUpd - 1) / kLineUpd;
-  const dim3 g((dm.nx + 1 + W - 1) / W, nseg, (D == 1 ? dm.nz : dm.ny) + 1);
-  const size_t smem = NodeTileSize<D, FIRST, LAST, K, W>::bytes;
-  auto kern = k_cyc_sweep_nodes_t<D, FIRST, LAST, K, R, W, GL>;
-  smem_opt_in((const void*)kern, smem);
-  kern<<<g, 32 * W, smem, s>>>(dm, a.S, a.ph, prev, a.x0, a.xl, a.vh, a.nm, udin, udout, a.dpf, a.Gd, a.st.mass, a.v,
-                               a.nm, a.vnorm, a.ecn);
-}
-
-template <int D, bool FIRST, bool LAST, int K, typename R>
-static void sweep_nodes_launch(const CycleArgs& a, int prev, const double* udin, double* udout, cudaStream_t s) {
-  const Dims& dm = a.dm;
-  const int nseg = (dm.ncd(D) + 1 + kLineUpd - 1) / kLineUpd;
-  const int T = 32 * kLineWarps;
-  // the generalised limiters (FP64) have their own kernels
-  const bool gl = sizeof(R) == 8 && a.ph.ordre_projection > 1 && a.ph.limiteur_id >= 3;
-  if constexpr (D == 0) {
-    const dim3 g(nseg, (dm.ny + 1 + kLineWarps - 1) / kLineWarps, dm.nz + 1);
-    if (gl)
-      k_cyc_sweep_nodes_x<FIRST, LAST, K, R, true><<<g, T, 0, s>>>(dm, a.S, a.ph, prev, a.x0, a.xl, a.vh, a.nm, udin,
-                                                                udout, a.dpf, a.Gd, a.st.mass, a.v, a.nm, a.vnorm, a.ecn);
-    else
-      k_cyc_sweep_nodes_x<FIRST, LAST, K, R><<<g, T, 0, s>>>(dm, a.S, a.ph, prev, a.x0, a.xl, a.vh, a.nm, udin, udout,
-                                                       a.dpf, a.Gd, a.st.mass, a.v, a.nm, a.vnorm, a.ecn);
-  } else {
-    if constexpr (sizeof(R) == 8) {
-      if (gl) { sweep_nodes_launch_w<D, FIRST, LAST, K, R, kLineWarps, true>(a, prev, udin, udout, s); return; }
-    }
-    // lines per block of this sweep (the tuning; K > 1 meshes keep 8)
-    const int w = K == 1 ? a.lines[BK_NODES_X + D] : kLineWarps;
-    if (w == 32) sweep_nodes_launch_w<D, FIRST, LAST, K, R, 32>(a, prev, udin, udout, s);
-    else if (w == 16) sweep_nodes_launch_w<D, FIRST, LAST, K, R, 16>(a, prev, udin, udout, s);
-    else sweep_nodes_launch_w<D, FIRST, LAST, K, R, 8>(a, prev, udin, udout, s);
-  }
-}
-
-// One node sweep along D of a mesh with K environments (dual mass fluxes in K planes).
-template <int D, int K, typename R>
-static void sweep_nodes_d(const CycleArgs& a, bool first, bool last, int prev, const double* udin, double* udout,
-                          cudaStream_t s) {
-  if (first) sweep_nodes_launch<D, true, false, K, R>(a, prev, udin, udout, s);
-  else if (last) sweep_nodes_launch<D, false, true, K, R>(a, prev, udin, udout, s);
-  else sweep_nodes_launch<D, false, false, K, R>(a, prev, udin, udout, s);
-}
-
-// R: evaluation precision of the sweep (double, or float in the mixed form).
-template <int K, typename R = double>
-static void sweep_nodes(const CycleArgs& a, int d, bool first, bool last, int prev, const double* udin,
-                        double* udout, cudaStream_t s) {
-  if (d == 0) sweep_nodes_d<0, K, R>(a, first, last, prev, udin, udout, s);
-  else if (d == 1) sweep_nodes_d<1, K, R>(a, first, last, prev, udin, udout, s);
-  else sweep_nodes_d<2, K, R>(a, first, last, prev, udin, udout, s);
-}
-
-
 }  // namespace mhy

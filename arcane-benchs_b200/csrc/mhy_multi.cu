@@ -25,6 +25,7 @@
 
 #include "mhy_lagrange.cuh"
 #include "mhy_line.cuh"
+#include "mhy_march.cuh"
 
 namespace mhy {
 
@@ -1191,10 +1192,18 @@ static void bat_env_nodes(const BatchPlan& P, int it, int prev, cudaStream_t s, 
   if constexpr (DD == 0)
     bat_env_launch(k_bat_env_nodes_x<FIRST, LAST, K, R, GL>, 32 * kLineWarps, 0, P, kind, kind, s, m, P.descs,
                    P.work[kind], P.nwork[kind], it, prev);
-  else
+  else {
+    if constexpr (sizeof(R) == 4 || FIRST) {
+      if (P.march[kind]) {
+        launch_march(k_bat_sweep_nodes_m<DD, FIRST, LAST, K, R, GL>, P, kind, s, m, P.descs, P.mwork[kind],
+                     P.nmwork[kind], prev, march_len(P.lines[kind]));
+        return;
+      }
+    }
     bat_env_launch(k_bat_env_nodes_t<DD, FIRST, LAST, K, R, GL>, 32 * kLineWarps,
                    NodeTileSize<DD, FIRST, LAST, K, kLineWarps>::bytes, P, kind, kind, s, m, P.descs, P.work[kind],
                    P.nwork[kind], it, prev);
+  }
 }
 
 template <int K, int DD, typename R, bool GL>

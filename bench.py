@@ -98,7 +98,7 @@ def parse():
 # on: after any change to those sources the figure is reported as stale (null).
 TRAFFIC_PER_CYCLE = {("sedov", 128, "fp64"): (3460821504.0, "1fee7bc5e6c8a96c"),
                      ("sedov", 128, "mixed"): (2910358272.0, "1fee7bc5e6c8a96c")}
-KERNEL_SOURCES = ("mhy_kernels.cuh", "mhy_device.cuh", "mhy_pow_third.h", "mhy_quot.h", "mhy_line.cuh", "mhy_lagrange.cuh",
+KERNEL_SOURCES = ("mhy_kernels.cuh", "mhy_device.cuh", "mhy_pow_third.h", "mhy_quot.h", "mhy_line.cuh", "mhy_march.cuh", "mhy_lagrange.cuh",
                   "mhy_kernels.cu", "mhy_cycle.cu", "mhy_multi.cu")
 
 
