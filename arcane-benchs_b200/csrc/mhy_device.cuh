@@ -74,7 +74,13 @@ __device__ __forceinline__ R dv(R x, R y, R r, unsigned* oor) {
   else if constexpr (SP) return quo_from_rcp(x, y, r, *oor);
   else return qdiv(x, y, r);
 }
-// A quotient with a denominator of its own.
+// x / y; in the speculative form with the branch-free quotient.
+template <typename R, bool SP>
+__device__ __forceinline__ R quo_of(R x, R y, unsigned* oor) {
+  if constexpr (sizeof(R) == 8 && SP) return quo_fast(x, y, *oor);
+  else return x / y;
+}
+// A quotient of the limiters: as quo_of, but FP32's fast division in the mixed form.
 template <typename R, bool SP>
 __device__ __forceinline__ R qu(R x, R y, unsigned* oor) {
   if constexpr (sizeof(R) == 4) return __fdividef(x, y);
@@ -94,10 +100,10 @@ template <typename R> __device__ __forceinline__ R tmax(R a, R b) { return (a < 
 // fluxLimiterG, mahyco/src/Remap/UtilesRemap.cc:127-175: the generalised
 // limiters for uneven widths (ids TypesMahyco.h:65-74: 3 minmodG, 4
 // superBeeG, 5 vanLeerG, 6 arithmeticG, 7 ultrabeeG), std::min / std::max.
-template <typename R>
+template <typename R, bool SP = false>
 __device__ __forceinline__ R flux_limiter_g(int id, R gradplus, R gradmoins, R y0, R yplus, R ymoins, R h0, R hplus,
-                                            R hmoins) {
-  const R zero = R(0), half = R(0.5);
+                                            R hmoins, unsigned* oor = nullptr) {
+  const R zero = R(0);
   R grady = zero;
   if (gradplus * gradmoins < zero) return zero;
   if (id == 3) {
@@ -107,21 +113,21 @@ __device__ __forceinline__ R flux_limiter_g(int id, R gradplus, R gradmoins, R y
     if ((yplus - ymoins) > zero) grady = tmax(fabs(gradplus), fabs(gradmoins));
     else grady = -tmax(fabs(gradplus), fabs(gradmoins));
   } else if (id == 5) {
-    const R lambdaplus = (h0 / R(2) + hplus) / (h0 + hplus + hmoins);
-    const R lambdamoins = (h0 / R(2) + hmoins) / (h0 + hplus + hmoins);
+    const R lambdaplus = quo_of<R, SP>(h0 / R(2) + hplus, h0 + hplus + hmoins, oor);
+    const R lambdamoins = quo_of<R, SP>(h0 / R(2) + hmoins, h0 + hplus + hmoins, oor);
     if ((lambdaplus * gradplus + lambdamoins * gradmoins) != zero)
-      grady = gradplus * gradmoins / (lambdaplus * gradplus + lambdamoins * gradmoins);
+      grady = quo_of<R, SP>(gradplus * gradmoins, lambdaplus * gradplus + lambdamoins * gradmoins, oor);
     else grady = zero;
   } else if (id == 7) {
-    grady = (yplus - ymoins) / h0;
+    grady = quo_of<R, SP>(yplus - ymoins, h0, oor);
   } else if (id == 6) {
-    const R lambdaplus = (h0 / R(2) + hplus) / (h0 + hplus + hmoins);
-    const R lambdamoins = (h0 / R(2) + hmoins) / (h0 + hplus + hmoins);
+    const R lambdaplus = quo_of<R, SP>(h0 / R(2) + hplus, h0 + hplus + hmoins, oor);
+    const R lambdamoins = quo_of<R, SP>(h0 / R(2) + hmoins, h0 + hplus + hmoins, oor);
     grady = lambdamoins * gradplus + lambdaplus * gradmoins;
   }
-  (void)half; (void)y0;
-  const R gradMplus = gradplus * (h0 + hplus) / h0;
-  const R gradMmoins = gradmoins * (h0 + hmoins) / h0;
+  (void)y0;
+  const R gradMplus = quo_of<R, SP>(gradplus * (h0 + hplus), h0, oor);
+  const R gradMmoins = quo_of<R, SP>(gradmoins * (h0 + hmoins), h0, oor);
   const R gradM = tmin(fabs(gradMplus), fabs(gradMmoins));
   if ((yplus - ymoins) > zero) grady = tmin(fabs(gradM), fabs(grady));
   else grady = -tmin(fabs(gradM), fabs(grady));

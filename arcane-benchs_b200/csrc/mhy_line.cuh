@@ -286,36 +286,68 @@ __device__ __forceinline__ void pb_fluxes(const Phys& ph, int type, double ppv, 
 // Order-3 face value of one variable (Remap-ordre-3.cc:7-131): y and h of
 // the six cells bbb, bb, b | f, ff, fff around the face (clamped at the ends
 // of the line) and u_f dt.
-__device__ __forceinline__ double o3_grad(double hm, double h0, double hp, double ym, double y0, double yp) {
-  return h0 / (hm + h0 + hp) * ((2. * hm + h0) / (h0 + hp) * (yp - y0) + (h0 + 2. * hp) / (hm + h0) * (y0 - ym));
+// The factors that depend on the widths and u_f dt only are formed once for all
+// variables (O3Coef); SP: with the quotients of mhy_quot.h.
+struct O3Coef {
+  double ga[4], gb[4], gc[4];              // the four gradients
+  double t1[3], ta[3], tb[3], w[3], z[3];  // the three interface values
+  double vdt, x1, x2, nm, np;              // 0.5 x / dx, 2/3 x / dx; (1 - num) / num, (1 + nup) / nup
+};
+template <bool SP>
+__device__ __forceinline__ O3Coef o3_coef(const double h[6], double vdt, unsigned* oor) {
+  O3Coef k;
+  auto quo = [&](double x, double y) { return quo_of<double, SP>(x, y, oor); };
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const double hm = h[g], h0 = h[g + 1], hp = h[g + 2];
+    k.ga[g] = quo(h0, hm + h0 + hp);
+    k.gb[g] = quo(2. * hm + h0, h0 + hp);
+    k.gc[g] = quo(h0 + 2. * hp, hm + h0);
+  }
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const double hmm = h[s], hm = h[s + 1], hp = h[s + 2], hpp = h[s + 3];
+    k.t1[s] = quo(2. * hp * hm, hm + hp) * (quo(hmm + hm, 2. * hm + hp) - quo(hpp + hp, 2. * hp + hm));
+    k.ta[s] = quo(-hm * (hmm + hm), 2. * hm + hp);
+    k.tb[s] = quo(hp * (hp + hpp), hm + 2. * hp);
+    k.w[s] = quo(hm, hm + hp);
+    k.z[s] = quo(1., hmm + hm + hp + hpp);
+  }
+  k.vdt = vdt;
+  k.x1 = k.x2 = k.nm = k.np = 0.;
+  if (vdt > 0. || vdt < 0.) {
+    const double x = vdt > 0. ? vdt : -vdt, dx = vdt > 0. ? h[2] : h[3];
+    k.x1 = quo(0.5 * x, dx);
+    k.x2 = quo(2. / 3. * x, dx);
+    const double num = quo(vdt, h[2]), nup = quo(vdt, h[3]);
+    k.nm = quo(1. - num, num);
+    k.np = quo(1. + nup, nup);
+  }
+  return k;
 }
-__device__ __forceinline__ double o3_ystar(double hmm, double hm, double hp, double hpp, double ymm, double ym,
-                                           double yp, double ypp, double gradm, double gradp) {
-  const double tmp1 = (2. * hp * hm) / (hm + hp) * ((hmm + hm) / (2. * hm + hp) - (hpp + hp) / (2. * hp + hm)) * (yp - ym);
-  const double tmp2 = -hm * (hmm + hm) / (2. * hm + hp) * gradp + hp * (hp + hpp) / (hm + 2. * hp) * gradm;
-  return ym + hm / (hm + hp) * (yp - ym) + 1. / (hmm + hm + hp + hpp) * (tmp1 + tmp2);
-}
-__device__ __forceinline__ double o3_flux(const double y[6], const double h[6], double vdt) {
-  const double ymmm = y[0], ymm = y[1], ym = y[2], yp = y[3], ypp = y[4], yppp = y[5];
-  const double hmmm = h[0], hmm = h[1], hm = h[2], hp = h[3], hpp = h[4], hppp = h[5];
-  const double gradmm = o3_grad(hmmm, hmm, hm, ymmm, ymm, ym);
-  const double gradm = o3_grad(hmm, hm, hp, ymm, ym, yp);
-  const double gradp = o3_grad(hm, hp, hpp, ym, yp, ypp);
-  const double gradpp = o3_grad(hp, hpp, hppp, yp, ypp, yppp);
-  const double ystarm = o3_ystar(hmmm, hmm, hm, hp, ymmm, ymm, ym, yp, gradmm, gradm);
-  const double ystar = o3_ystar(hmm, hm, hp, hpp, ymm, ym, yp, ypp, gradm, gradp);
-  const double ystarp = o3_ystar(hm, hp, hpp, hppp, ym, yp, ypp, yppp, gradp, gradpp);
-  const double ym_m = ystarm, ym_p = ystar, yp_m = ystar, yp_p = ystarp;
+__device__ __forceinline__ double o3_value(const O3Coef& k, const double y[6]) {
+  double grad[4], ystar[3];
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    grad[g] = k.ga[g] * (k.gb[g] * (y[g + 2] - y[g + 1]) + k.gc[g] * (y[g + 1] - y[g]));
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const double ym = y[s + 1], yp = y[s + 2];
+    const double tmp1 = k.t1[s] * (yp - ym);
+    const double tmp2 = k.ta[s] * grad[s + 1] + k.tb[s] * grad[s];
+    ystar[s] = ym + k.w[s] * (yp - ym) + k.z[s] * (tmp1 + tmp2);
+  }
+  const double ymm = y[1], ym = y[2], yp = y[3], ypp = y[4], vdt = k.vdt;
+  const double ym_m = ystar[0], ym_p = ystar[1], yp_m = ystar[1], yp_p = ystar[2];
   const double grad_m = ym_p - ym_m, grad_p = yp_p - yp_m;
   const double ym6 = 6. * (ym - 0.5 * (ym_m + ym_p));
   const double yp6 = 6. * (yp - 0.5 * (yp_m + yp_p));
   double flux;
-  if (vdt > 0.) { const double x = vdt, dx = hm; flux = ym_p - 0.5 * x / dx * (grad_m - (1. - 2. / 3. * x / dx) * ym6); }
-  else if (vdt < 0.) { const double x = -vdt, dx = hp; flux = yp_m + 0.5 * x / dx * (grad_p - (1. - 2. / 3. * x / dx) * yp6); }
+  if (vdt > 0.) flux = ym_p - k.x1 * (grad_m - (1. - k.x2) * ym6);
+  else if (vdt < 0.) flux = yp_m + k.x1 * (grad_p - (1. - k.x2) * yp6);
   else return 0.;
-  const double num = vdt / hm, nup = vdt / hp;
-  const double ym_ym = ym + (1. - num) / num * (ym - ymm);
-  const double yp_ym = yp - (1. + nup) / nup * (yp - ypp);
+  const double ym_ym = ym + k.nm * (ym - ymm);
+  const double yp_ym = yp - k.np * (yp - ypp);
   const double i10 = amin(ym, yp), i11 = amax(ym, yp);
   double i20, i21;
   if (vdt >= 0.) { i20 = amin(ym, ym_ym); i21 = amax(ym, ym_ym); }
@@ -415,6 +447,7 @@ __device__ __forceinline__ void cell_line(const Phys& ph, double dt, const Scala
   } else if constexpr (GL) {
     // generalised limiters (RemapADIService.cc:319-437 -> UtilesRemap.cc:295-330):
     // back and front cells are the cell itself at the ends of the line
+    unsigned go = 0u;                                     // lanes 1..30: what reaches an updated cell
     R Pn[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) Pn[v] = __shfl_down_sync(full, P[v], 1);
@@ -422,7 +455,8 @@ __device__ __forceinline__ void cell_line(const Phys& ph, double dt, const Scala
     const R h0 = (R)in.h, hm = (R)(inner ? hb : in.h), hp = (R)(infr ? hn : in.h);
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      G[v] = flux_limiter_g<R>(lim, gr[v], g[v], P[v], infr ? Pn[v] : P[v], inner ? Pp[v] : P[v], h0, hp, hm);
+      G[v] = flux_limiter_g<R, SP>(lim, gr[v], g[v], P[v], infr ? Pn[v] : P[v], inner ? Pp[v] : P[v], h0, hp, hm, &go);
+    if constexpr (SP) { const int lane = threadIdx.x & 31; if (valid && lane >= 1 && lane <= 30) *oor |= go; }
   } else {
     // only the gradients of lanes 1..30 reach an updated cell
     unsigned go = 0u;
@@ -589,12 +623,14 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
       for (int c = 0; c < 3; ++c) G[c] = R(0);
       if (valid && inner) {
         const R h0 = (R)(0.5 * (xp - xm));
+        unsigned go = 0u;                             // lanes 1..30: what reaches an updated node
         R hmo, hpl;
         if (!bb_ok) { hmo = R(0); hpl = (R)(0.5 * (xp2 - x)); }
         else if (!ff_ok) { hpl = R(0); hmo = (R)(0.5 * (x - xm2)); }
         else { hmo = (R)(0.5 * (x - xm2)); hpl = (R)(0.5 * (xp2 - x)); }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) G[c] = flux_limiter_g<R>(lim, gf[c], gb[c], P[c], Pp[c], Pm[c], h0, hpl, hmo);
+        for (int c = 0; c < 3; ++c) G[c] = flux_limiter_g<R, SP>(lim, gf[c], gb[c], P[c], Pp[c], Pm[c], h0, hpl, hmo, &go);
+        if constexpr (SP) { if (lane >= 1 && lane <= 30) *oor |= go; }
       }
     } else if (valid && inner) {
       unsigned go = 0u;                               // lanes 1..30: what reaches an updated node

@@ -205,7 +205,7 @@ __device__ __forceinline__ void nodes_march(const CycleArgs& A, int prev_inner, 
           else { hmo = (R)(0.5 * (xw[s2] - xb2)); hpl = (R)(0.5 * (xp2 - xw[s2])); }
 #pragma unroll
           for (int c = 0; c < 3; ++c)
-            G[s2][c] = flux_limiter_g<R>(lim, g[s2][c], g[s1][c], P[s2][c], P[s3][c], P[s1][c], h0, hpl, hmo);
+            G[s2][c] = flux_limiter_g<R, SP>(lim, g[s2][c], g[s1][c], P[s2][c], P[s3][c], P[s1][c], h0, hpl, hmo, oor);
         } else {
           limited_slopes<3, R, true, SP, true>(lim, g[s1], g[s2], G[s2], oor);
         }

@@ -581,6 +581,7 @@ __device__ __forceinline__ void o3_faces_env_item(const Dims& dm, const Scalars*
   const long long tf = dm.fid(D, i, j, k) - (D == 0 ? 0 : (D == 1 ? dm.Fx : dm.Fx + dm.Fy));
   const double vdt = fd.u[D][tf] * S->dt;
   double pf[NV];
+  const O3Coef k3 = o3_coef<false>(h, vdt, nullptr);
   double pb[NV], pn[NV];                              // Phi of the two cells of the face
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -588,7 +589,7 @@ __device__ __forceinline__ void o3_faces_env_item(const Dims& dm, const Scalars*
 #pragma unroll
     for (int a = 0; a < 6; ++a) y[a] = qdiv(Uin[v * C + cc[a]], den[a], rden[a]);
     pb[v] = y[2]; pn[v] = y[3];
-    pf[v] = o3_flux(y, h, vdt);
+    pf[v] = o3_value(k3, y);
   }
   const uint32_t codeb = FIRST ? fd.est[cc[2]] : est_code<K>(pb);
   const uint32_t codef = FIRST ? fd.est[cc[3]] : est_code<K>(pn);
