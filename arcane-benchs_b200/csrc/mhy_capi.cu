@@ -736,8 +736,8 @@ std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int or
   for (int i = 0; i < n; ++i) {
     int gx, gy, gz;
     if (kind == kColumns) {
-      size_t smem;
-      batch_column_shape(inst[i]->dm, gx, gy, smem);
+      int strip;
+      batch_column_shape(inst[i]->dm, gx, gy, strip);
       gz = 1;
     } else {
       batch_work_shape(inst[i]->dm, kind, lines, march, gx, gy, gz);
@@ -843,10 +843,9 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
     b->plan.cwork = b->d_cwork;
     b->plan.ncwork = (int)w.size();
     for (const mhy_ctx* c : b->inst) {
-      int blocks, segments;
-      size_t smem;
-      batch_column_shape(c->dm, blocks, segments, smem);
-      b->plan.col_smem = std::max(b->plan.col_smem, smem);
+      int blocks, segments, strip;
+      batch_column_shape(c->dm, blocks, segments, strip);
+      b->plan.col_strip = std::max(b->plan.col_strip, strip);
     }
   }
   err = cudaMalloc(&b->d_descs, n * sizeof(CycleArgs));

@@ -897,10 +897,10 @@ int persistent_grid(const void* kernel, int threads, size_t smem, int nwork, int
   return persistent_blocks(kernel, threads, smem, nwork, pct);
 }
 
-void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem) {
+void batch_column_shape(const Dims& dm, int& blocks, int& segments, int& strip) {
   blocks = col_blocks(dm.nx, dm.ny);
   segments = col_segments(dm.nx, dm.ny, dm.nz);
-  smem = col_smem(dm.nx);
+  strip = col_strip(dm.nx);
 }
 
 // The y/z sweeps of a batch with a table of marching work (FP64 node sweeps
@@ -1071,8 +1071,8 @@ void launch_batch_cycle(const BatchPlan& P, int sens, cudaStream_t s, KernelMark
     auto kern = P.precision ? k_bat_lagrange_cells<1, float, false, false>
                             : (hc ? k_bat_lagrange_cells<1, double, true, true> : k_bat_lagrange_cells<1, double, false, true>);
     launch_persistent(kern, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  } else if (hc) launch_bat_columns(k_bat_lagrange_columns<1, true>, P, s, m);
-  else launch_bat_columns(k_bat_lagrange_columns<1, false>, P, s, m);
+  } else if (hc) launch_bat_columns<1, true>(P, s, m);
+  else launch_bat_columns<1, false>(P, s, m);
   launch_bat_csts_forward(P, s);   // PrepareRemap.cc:456, then the face velocities
   if (P.precision) bat_sweeps<float, false>(P, sens, s, m);
   else if (P.gl) bat_sweeps<double, true>(P, sens, s, m);

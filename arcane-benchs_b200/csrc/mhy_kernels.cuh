@@ -165,7 +165,7 @@ struct BatchPlan {
   int csts;                     // every instance takes schema-csts (FP64)
   const int4* cwork;            // the Lagrange cell kernel's columns (instance, chunk, segment); not schema-csts
   int ncwork;
-  size_t col_smem;              // its shared memory, the largest instance's
+  int col_strip;                // the longest strip of nodes its instances need
   const int4* fwork;            // schema-csts: face work table (instance, chunk of 128 faces of all directions)
   int nfwork;
   const int4* o3work[3];        // order 3: face work tables (instance, chunk of 128 faces) per direction
@@ -183,7 +183,7 @@ struct KernelMarks {
 // Blocks of one instance's grid for a kernel kind; march: its y/z sweep marches (BatchPlan::march).
 void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, int& gy, int& gz);
 bool batch_marches(const CycleArgs& a, int kind, long long nodes);
-void batch_column_shape(const Dims& dm, int& blocks, int& segments, size_t& smem);
+void batch_column_shape(const Dims& dm, int& blocks, int& segments, int& strip);
 // Dynamic shared memory above the default 48 KB needs an opt-in per kernel and device.
 void smem_opt_in(const void* kernel, size_t bytes);
 // Records an event after a launch (autotuning): slot `kind` of the marks.
@@ -224,6 +224,24 @@ __global__ void k_dt_min(Dims dm, Scalars* S, const double* L, const double* cs,
 dim3 cell_grid(const Dims& dm, int& linear);
 __global__ void k_dt_finish(Scalars* S, Phys ph);
 __global__ void k_dt_finish_ext(Scalars* S, Phys ph, const unsigned long long* min_bits);
+
+// Columns: a block takes kColThreads consecutive cells of one z layer (x
+// fastest) and a segment of layers.  Blocks of a layer, and segments: kColLayers
+// layers each; short columns of small meshes are cut finer so that the blocks
+// fill the chip (3 blocks on 148 SMs).
+constexpr int kColThreads = 128;
+constexpr int kColLayers = 8;
+__host__ __device__ __forceinline__ int col_blocks(int nx, int ny) { return (nx * ny + kColThreads - 1) / kColThreads; }
+__host__ __device__ __forceinline__ int col_segments(int nx, int ny, int nz) {
+  const int by_len = (nz + kColLayers - 1) / kColLayers, fill = (444 + col_blocks(nx, ny) - 1) / col_blocks(nx, ny);
+  const int want = fill < nz ? fill : nz;
+  return by_len > want ? by_len : want;
+}
+__host__ __device__ __forceinline__ void col_layers(int nx, int ny, int nz, int seg, int& k0, int& k1) {
+  const int nseg = col_segments(nx, ny, nz);
+  k0 = (int)((long long)nz * seg / nseg);
+  k1 = (int)((long long)nz * (seg + 1) / nseg);
+}
 
 // computeHydroDeltaT (MahycoModule.cc:2047-2061): min over cells of
 // L / (c + max |v|) (|v| per node precomputed), warp shuffle + block

@@ -534,29 +534,24 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_cyc_lagrange_ce
 // block instead of once for each of its 8 cells.  The cell's own state and the
 // normals of its faces are copied at the start of its layer and used at its end.
 // Bound: FP64 latency with 12 warps an SM (168 registers hold the corner
-// vectors' sums; the FP64 pipe is 46 % busy, its work alone takes 150 us and the
-// bytes 165 us on Sedov 128^3).  Measured on B200 against one thread a cell with
-// the nodes gathered from memory: 323 -> 307-315 us there (428 -> 48 bytes of
-// spills), 1372 -> 1156-1233 us on a batch of 24 meshes 32^3..96^3, 868 ->
-// 807-850 us with two gases on 256x128x128.
-constexpr int kColThreads = 128;
-constexpr int kColLayers = 8;        // layers a segment
+// vectors' sums; the FP64 work alone takes 150 us and the bytes 165 us on Sedov
+// 128^3).  Measured on B200 against one thread a cell with the nodes gathered
+// from memory: 323 -> 249 us there (315 us with strips of a length known at run
+// time only), 1372 -> 1100 us on a batch of 24 meshes 32^3..96^3, 868 -> 665 us
+// with two gases on 256x128x128.
 constexpr int kColPriv = 24;         // doubles a cell: 18 normals (low and high faces), 6 state values
 
 // Nodes of a strip: a plane of nodes comes as two strips, from the low row of
 // the block's first cell onwards and from one row up; a strip holds the block's
-// cells, one node more a row that it touches and one for its last cell.
-__host__ __device__ __forceinline__ int col_strip(int nx) { return kColThreads + (kColThreads + nx - 2) / nx + 2; }
-__host__ __device__ __forceinline__ size_t col_smem(int nx) {
-  return (size_t)(3 * 12 * col_strip(nx) + kColPriv * kColThreads) * sizeof(double);
+// cells, one node more a row that it touches and one for its last cell.  Two
+// lengths, known at compile time so that a cell's nodes lie at fixed offsets:
+// one for rows of 26 cells and more, one for any row of two cells and more.
+constexpr int kColStrip = 136, kColStripWide = 200;
+__host__ __device__ __forceinline__ int col_strip(int nx) {
+  return kColThreads + (kColThreads + nx - 2) / nx + 2 <= kColStrip ? kColStrip : kColStripWide;
 }
-// Blocks of a layer and segments of the column; short columns of small meshes
-// are cut finer so that the blocks fill the chip (3 blocks on 148 SMs).
-__host__ __device__ __forceinline__ int col_blocks(int nx, int ny) { return (nx * ny + kColThreads - 1) / kColThreads; }
-__host__ __device__ __forceinline__ int col_segments(int nx, int ny, int nz) {
-  const int by_len = (nz + kColLayers - 1) / kColLayers, fill = (444 + col_blocks(nx, ny) - 1) / col_blocks(nx, ny);
-  const int want = fill < nz ? fill : nz;
-  return by_len > want ? by_len : want;
+__host__ __device__ __forceinline__ size_t col_smem(int strip) {
+  return (size_t)(3 * 12 * strip + kColPriv * kColThreads) * sizeof(double);
 }
 
 __device__ __forceinline__ void cp_async8(double* s, const double* g) {
@@ -565,16 +560,16 @@ __device__ __forceinline__ void cp_async8(double* s, const double* g) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
 template <int Left> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(Left) : "memory"); }
 
-template <int K, bool HC>
+template <int K, bool HC, int strip>
 __device__ __forceinline__ void lagrange_columns(const CycleArgs& A, int bx, int seg) {
   extern __shared__ double col_mem[];
   const Dims& dm = A.dm;
   const int nx = dm.nx, ny = dm.ny, nz = dm.nz, nnx = nx + 1, np = nnx * (ny + 1);
-  const int strip = col_strip(nx), tid = threadIdx.x;
+  const int tid = threadIdx.x;
   const int N = (int)dm.N, C = (int)dm.C, F = (int)dm.F;
   double* const priv = col_mem + 36 * strip;                      // [kColPriv][kColThreads]
-  const int nseg = col_segments(nx, ny, nz);
-  const int k0 = (int)((long long)nz * seg / nseg), k1 = (int)((long long)nz * (seg + 1) / nseg);
+  int k0, k1;
+  col_layers(nx, ny, nz, seg, k0, k1);
   const int p0 = bx * kColThreads, p = p0 + tid;
   const bool cell = p < nx * ny;
   const int i = p % nx, j = p / nx;
@@ -690,16 +685,16 @@ __device__ __forceinline__ void lagrange_columns(const CycleArgs& A, int bx, int
   }
 }
 
-template <int K, bool HC = false>
-__global__ void __launch_bounds__(kColThreads, 3) k_cyc_lagrange_columns(const __grid_constant__ CycleArgs a) {
-  lagrange_columns<K, HC>(a, blockIdx.x, blockIdx.y);
+template <int K, bool HC, int STRIP>
+__global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_cyc_lagrange_columns(const __grid_constant__ CycleArgs a) {
+  lagrange_columns<K, HC, STRIP>(a, blockIdx.x, blockIdx.y);
 }
 
 // The same over a batch's column table (instance, chunk, segment).  The
 // instance's arguments are read from shared memory where they are used:
 // fifty pointers in registers would spill.
-template <int K, bool HC = false>
-__global__ void __launch_bounds__(kColThreads, 3) k_bat_lagrange_columns(const CycleArgs* __restrict__ D,
+template <int K, bool HC, int STRIP>
+__global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat_lagrange_columns(const CycleArgs* __restrict__ D,
                                                                          const int4* __restrict__ W, int nw) {
   __shared__ CycleArgs a;
   for (int w = blockIdx.x; w < nw; w += gridDim.x) {
@@ -709,7 +704,7 @@ __global__ void __launch_bounds__(kColThreads, 3) k_bat_lagrange_columns(const C
     for (int x = threadIdx.x; x < (int)(sizeof(CycleArgs) / sizeof(double)); x += kColThreads)
       reinterpret_cast<double*>(&a)[x] = reinterpret_cast<const double*>(D + t.x)[x];
     __syncthreads();
-    lagrange_columns<K, HC>(a, t.y, t.z);
+    lagrange_columns<K, HC, STRIP>(a, t.y, t.z);
   }
 }
 
@@ -718,20 +713,23 @@ __global__ void __launch_bounds__(kColThreads, 3) k_bat_lagrange_columns(const C
 // 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1).
 constexpr long long kColMinCells = 65536;
 
-template <class Kern>
-static void launch_columns(Kern kern, const CycleArgs& a, cudaStream_t s) {
+template <int K, bool HC>
+static void launch_columns(const CycleArgs& a, cudaStream_t s) {
   const Dims& dm = a.dm;
-  const size_t smem = col_smem(dm.nx);
+  const int strip = col_strip(dm.nx);
+  const size_t smem = col_smem(strip);
+  auto kern = strip == kColStrip ? k_cyc_lagrange_columns<K, HC, kColStrip> : k_cyc_lagrange_columns<K, HC, kColStripWide>;
   smem_opt_in((const void*)kern, smem);
   kern<<<dim3(col_blocks(dm.nx, dm.ny), col_segments(dm.nx, dm.ny, dm.nz)), kColThreads, smem, s>>>(a);
 }
+
 // The cell kernel of a context, all but schema-csts.
 template <int K>
 static void launch_cells(const CycleArgs& a, cudaStream_t s) {
   const bool hc = a.fd.h != nullptr;               // cell widths: order 3 or the generalised limiters
   if (!a.ph.precision && a.dm.C >= kColMinCells) {
-    if (hc) launch_columns(k_cyc_lagrange_columns<K, true>, a, s);
-    else launch_columns(k_cyc_lagrange_columns<K, false>, a, s);
+    if (hc) launch_columns<K, true>(a, s);
+    else launch_columns<K, false>(a, s);
     return;
   }
   int linear;
@@ -741,12 +739,14 @@ static void launch_cells(const CycleArgs& a, cudaStream_t s) {
                            a.cqs, a.cqs32, a.L, a.U[0], a.xc, a.fd, a.env, a.Vlag, linear);
 }
 
-template <class Kern>
-static void launch_bat_columns(Kern kern, const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
-  smem_opt_in((const void*)kern, P.col_smem);
+template <int K, bool HC>
+static void launch_bat_columns(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  const size_t smem = col_smem(P.col_strip);
+  auto kern = P.col_strip == kColStrip ? k_bat_lagrange_columns<K, HC, kColStrip> : k_bat_lagrange_columns<K, HC, kColStripWide>;
+  smem_opt_in((const void*)kern, smem);
   if (P.ncwork > 0)
-    kern<<<persistent_grid((const void*)kern, kColThreads, P.col_smem, P.ncwork, P.occ_pct[BK_LCELLS]), kColThreads,
-           P.col_smem, s>>>(P.descs, P.cwork, P.ncwork);
+    kern<<<persistent_grid((const void*)kern, kColThreads, smem, P.ncwork, P.occ_pct[BK_LCELLS]), kColThreads, smem, s>>>(
+        P.descs, P.cwork, P.ncwork);
   mark(m, BK_LCELLS, s);
 }
 

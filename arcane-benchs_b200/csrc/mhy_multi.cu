@@ -1250,7 +1250,7 @@ static void batch_cycle_env(const BatchPlan& P, int sens, cudaStream_t s, Kernel
     }
   }
   if (!done) {
-    if constexpr (sizeof(R) == 8) launch_bat_columns(k_bat_lagrange_columns<K, HC>, P, s, m);
+    if constexpr (sizeof(R) == 8) launch_bat_columns<K, HC>(P, s, m);
     else bat_env_launch(k_bat_lagrange_cells<K, float, false, false>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
                         P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
   }
