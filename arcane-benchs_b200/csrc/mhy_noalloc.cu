@@ -10,15 +10,16 @@
 //
 // The reduction needs scratch memory (one partial minimum per block of the
 // first pass).  Here that scratch is a file-scope __device__ array, so the
-// entry point allocates nothing: it issues two kernel launches on the caller's
-// stream and returns.
+// entry point allocates nothing: it issues one or two kernel launches on the
+// caller's stream and returns.
 //
 // Limits and sharing, stated for users:
 //  * the scratch holds kNoAllocBlocks partial minima (64 KiB per GPU, kept by
 //    every GPU that loads this library until the process exits);
-//  * the first pass uses at most kNoAllocBlocks blocks of 256 threads and each
-//    thread takes at most kNoAllocCellsPerThread cells, so meshes are limited
-//    to kNoAllocMaxCells cells; larger meshes are rejected with MHY_ERR_ARG;
+//  * the first pass uses at most kNoAllocBlocks blocks of 256 threads; meshes
+//    are limited to kNoAllocMaxCells cells (64 a thread), larger ones are
+//    rejected with MHY_ERR_ARG.  Small meshes take one launch, which leaves the
+//    scratch alone;
 //  * every call on a device shares the same scratch and leaves its partial
 //    minima there; each call writes every slot it reads before reading it, so
 //    nothing has to be cleared, but calls that overlap on the GPU (different
@@ -37,6 +38,7 @@
 //    2152-2159).  The context's own reduction raises MHY_STATUS_NAN_DT for the
 //    same cells.
 #include <cuda.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -50,6 +52,9 @@ constexpr int kNoAllocBlocks = 8192;
 constexpr int kNoAllocThreads = 256;
 constexpr int kNoAllocCellsPerThread = 64;
 constexpr long long kNoAllocMaxCells = (long long)kNoAllocBlocks * kNoAllocThreads * kNoAllocCellsPerThread;
+constexpr int kNoAllocLayers = 4;                   // a segment's layers on meshes that do not fill the chip
+constexpr int kNoAllocCluster = 8;                  // blocks of the portable cluster size
+constexpr int kNoAllocClusterThreads = 1024;
 constexpr unsigned long long kDblMaxBits = 0x7fefffffffffffffull;
 // A block's partial minimum is the bit pattern of a non-negative double (bit
 // 63 clear); bit 63 set records that the block met an invalid cell.
@@ -113,42 +118,135 @@ __device__ __forceinline__ unsigned long long block_min(unsigned long long best,
   return best;  // valid in thread 0
 }
 
-// First pass: dx_sound = L / (c + max over the cell's nodes of |v|), as in
-// computeHydroDeltaT (mahyco/src/MahycoModule.cc:2047-2060); one partial
-// minimum per block (bit patterns of non-negative doubles order like
-// integers), with kInvalidBit set when the block met a NaN or negative value.
-__global__ void k_dt_partial_noalloc(Dims dm, const double* __restrict__ L, const double* __restrict__ cs,
-                                     const double* __restrict__ v, unsigned long long* __restrict__ scratch) {
+// computeHydroDeltaT (MahycoModule.cc:2047-2060) over the cells (p, k0..k1) of
+// one column: min of L / (c + max over the cell's nodes of |v|) as the bit
+// pattern of a non-negative double (they order like integers); invalid is set
+// where a value is NaN or negative.  The maximum is taken over |v|^2, in the
+// cell-node order, with one root a cell: the root is monotonic, so its result
+// is the maximum of the roots.  The four nodes of a layer's top are the next
+// layer's bottom.  Four layers are loaded before the first root and division,
+// whose branches would keep the loads apart.
+__device__ __forceinline__ unsigned long long column_dt_min(const Dims& dm, const double* __restrict__ L,
+                                                            const double* __restrict__ cs,
+                                                            const double* __restrict__ v, int p, int k0, int k1,
+                                                            bool& invalid) {
+  unsigned long long best = kDblMaxBits;
+  const int nx = dm.nx, nnx = nx + 1, np = nnx * (dm.ny + 1), layer = nx * dm.ny;
+  const int n0 = p + p / nx;                        // node (i, j) of the plane
+  const long long N = dm.N;
+  auto speed2 = [&](int n) {                         // the operations of |v| up to the root
+    const double x = v[n], y = v[N + n], z = v[2 * N + n];
+    return x * x + y * y + z * z;
+  };
+  auto plane = [&](int k, double* s) {
+    const int n = n0 + np * k;
+    s[0] = speed2(n); s[1] = speed2(n + 1); s[2] = speed2(n + nnx + 1); s[3] = speed2(n + nnx);
+  };
+  double b[4];
+  plane(k0, b);
+  for (int k = k0; k < k1; k += 4) {
+    double vmax[4], lc[4], cc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int kq = k + q < k1 ? k + q : k1 - 1;   // past the end the last cell again
+      double t[4];
+      plane(kq + 1, t);
+      lc[q] = L[p + layer * kq];
+      cc[q] = cs[p + layer * kq];
+      vmax[q] = 0.;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) vmax[q] = amax(b[a], vmax[q]);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) vmax[q] = amax(t[a], vmax[q]);
+      if (k + q + 1 < k1) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) b[a] = t[a];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double dx_sound = lc[q] / (cc[q] + sqrt(vmax[q]));
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(dx_sound);
+      if (dx_sound >= 0.) best = bits < best ? bits : best;
+      else invalid = true;
+    }
+  }
+  return best;
+}
+
+// The new dt of computeDeltaT (MahycoModule.cc:2144-2150) from the minimum:
+// min(cfl * min, 1.05 * dt_old, deltat_max); NaN and 0 after an invalid cell.
+__device__ __forceinline__ void write_dt(unsigned long long best, bool bad, double cfl, double dt_old,
+                                         double deltat_max, double* __restrict__ out) {
+  if (bad) {
+    out[0] = __longlong_as_double(0x7ff8000000000000ll);     // quiet NaN: no valid minimum
+    out[1] = 0.;
+    return;
+  }
+  const double minimum_aux = __longlong_as_double((long long)best);
+  double new_dt = cfl * minimum_aux;
+  new_dt = amin(new_dt, 1.05 * dt_old);
+  new_dt = amin(new_dt, deltat_max);
+  out[0] = minimum_aux;
+  out[1] = new_dt;
+}
+
+// The minimum over this block's part of the mesh (valid in thread 0), with
+// kInvalidBit set when the block met a NaN or negative value.  A thread walks
+// segments of `layers` layers of a column, a grid apart.
+__device__ __forceinline__ unsigned long long block_partial(const Dims& dm, const double* __restrict__ L,
+                                                            const double* __restrict__ cs,
+                                                            const double* __restrict__ v, int layers) {
   __shared__ unsigned long long wmin[32];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
   unsigned long long best = kDblMaxBits;
   bool invalid = false;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < dm.C;
-       c += (long long)gridDim.x * blockDim.x) {
-    int i, j, k; dm.cijk(c, i, j, k);
-    double vmax = 0.;
-    for (int a = 0; a < 8; ++a) {
-      long long n = dm.nid(i + kCellNodeOff[a][0], j + kCellNodeOff[a][1], k + kCellNodeOff[a][2]);
-      vmax = amax(norm2(d3(v[n], v[dm.N + n], v[2 * dm.N + n])), vmax);
-    }
-    double dx_sound = L[c] / (cs[c] + vmax);
-    if (dx_sound >= 0.) {
-      unsigned long long b = (unsigned long long)__double_as_longlong(dx_sound);
-      best = b < best ? b : best;
-    } else {
-      invalid = true;                               // NaN or negative
-    }
+  // (column, segment), columns fastest; kNoAllocMaxCells keeps the counts in 32 bits
+  const unsigned points = (unsigned)dm.nx * dm.ny, items = points * (unsigned)((dm.nz + layers - 1) / layers);
+  for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < items; w += gridDim.x * blockDim.x) {
+    const int seg = (int)(w / points), p = (int)(w - seg * points), k0 = seg * layers;
+    const int k1 = k0 + layers < dm.nz ? k0 + layers : dm.nz;
+    const unsigned long long b = column_dt_min(dm, L, cs, v, p, k0, k1, invalid);
+    best = b < best ? b : best;
   }
   if (invalid) bad = 1;                             // benign race: every writer stores 1
   best = block_min(best, wmin);                     // its barrier also orders the writes to `bad`
-  if (threadIdx.x == 0) scratch[blockIdx.x] = best | (bad ? kInvalidBit : 0ull);
+  return bad ? best | kInvalidBit : best;
 }
 
-// Second pass: minimum of the partial minima, then the new dt of
-// computeDeltaT (MahycoModule.cc:2144-2150): min(cfl * min, 1.05 * dt_old, deltat_max);
-// NaN and 0 when any block met an invalid cell.
+// First pass: one partial minimum per block.
+__global__ void __launch_bounds__(kNoAllocThreads) k_dt_partial_noalloc(Dims dm, const double* __restrict__ L,
+    const double* __restrict__ cs, const double* __restrict__ v, int layers, unsigned long long* __restrict__ scratch) {
+  const unsigned long long best = block_partial(dm, L, cs, v, layers);
+  if (threadIdx.x == 0) scratch[blockIdx.x] = best;
+}
+
+// The whole call on one cluster: its first block gathers the partial minima in
+// its shared memory.
+__global__ void __launch_bounds__(kNoAllocClusterThreads) k_dt_cluster_noalloc(Dims dm, const double* __restrict__ L,
+    const double* __restrict__ cs, const double* __restrict__ v, double cfl, double dt_old, double deltat_max,
+    double* __restrict__ out) {
+  __shared__ unsigned long long part[kNoAllocCluster];
+  auto cluster = cooperative_groups::this_cluster();
+  cluster.barrier_arrive();                         // this block runs
+  unsigned long long best = block_partial(dm, L, cs, v, kNoAllocLayers);
+  cluster.barrier_wait();                           // every block runs, so its shared memory is there
+  if (threadIdx.x == 0) cluster.map_shared_rank(part, 0)[blockIdx.x] = best;
+  cluster.sync();
+  if (blockIdx.x || threadIdx.x) return;
+  unsigned long long bad = 0ull;
+  best = kDblMaxBits;
+  for (unsigned b = 0; b < kNoAllocCluster; ++b) {
+    const unsigned long long m = part[b] & ~kInvalidBit;
+    bad |= part[b] & kInvalidBit;
+    best = m < best ? m : best;
+  }
+  write_dt(best, bad != 0ull, cfl, dt_old, deltat_max, out);
+}
+
+// Second pass: minimum of the partial minima, then the new dt.
 __global__ void k_dt_final_noalloc(const unsigned long long* __restrict__ scratch, int nparts, double cfl,
                                    double dt_old, double deltat_max, double* __restrict__ out) {
   __shared__ unsigned long long wmin[32];
@@ -165,19 +263,7 @@ __global__ void k_dt_final_noalloc(const unsigned long long* __restrict__ scratc
   }
   if (invalid) bad = 1;
   best = block_min(best, wmin);
-  if (threadIdx.x == 0) {
-    if (bad) {
-      out[0] = __longlong_as_double(0x7ff8000000000000ll);   // quiet NaN: no valid minimum
-      out[1] = 0.;
-      return;
-    }
-    const double minimum_aux = __longlong_as_double((long long)best);
-    double new_dt = cfl * minimum_aux;
-    new_dt = amin(new_dt, 1.05 * dt_old);
-    new_dt = amin(new_dt, deltat_max);
-    out[0] = minimum_aux;
-    out[1] = new_dt;
-  }
+  if (threadIdx.x == 0) write_dt(best, bad, cfl, dt_old, deltat_max, out);
 }
 
 }  // namespace
@@ -214,10 +300,32 @@ extern "C" int mhy_compute_hydro_dt_noalloc(int32_t nx, int32_t ny, int32_t nz, 
     scratch = sa.addr;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  long long want = (dm.C + kNoAllocThreads - 1) / kNoAllocThreads;
-  const int nblocks = (int)(want < kNoAllocBlocks ? want : kNoAllocBlocks);
-  k_dt_partial_noalloc<<<nblocks, kNoAllocThreads, 0, s>>>(dm, L, cs, v, scratch);
-  k_dt_final_noalloc<<<1, 1024, 0, s>>>(scratch, nblocks, cfl, dt_old, deltat_max, out);
+  // One cluster of eight blocks where it has a thread for every segment of 4
+  // layers: a second launch costs more than eight SMs lose.  Otherwise segments
+  // of 8 layers, of 4 where those would not fill the chip (148 SMs x 8 blocks).
+  // Measured on B200, the call, against one thread a cell with its eight nodes in
+  // two launches: 100x5x5 11.9 -> 9.0 us, 32^3 11.9 -> 8.9 (two segments a thread,
+  // 40^3: 13.6 against 11.9 in two launches), 64^3 14.3 -> 11.9, 128^3 66 -> 37.
+  const long long points = (long long)nx * ny, segments = points * ((nz + kNoAllocLayers - 1) / kNoAllocLayers);
+  if (segments <= kNoAllocCluster * kNoAllocClusterThreads) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kNoAllocCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kNoAllocCluster);
+    cfg.blockDim = dim3((unsigned)((segments + 32 * kNoAllocCluster - 1) / (32 * kNoAllocCluster)) * 32);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_dt_cluster_noalloc, dm, L, cs, v, cfl, dt_old, deltat_max, out);
+  } else {
+    const int layers = points * ((nz + 7) / 8) < 148LL * 8 * kNoAllocThreads ? kNoAllocLayers : 8;
+    const long long want = (points * ((nz + layers - 1) / layers) + kNoAllocThreads - 1) / kNoAllocThreads;
+    const int nblocks = (int)(want < kNoAllocBlocks ? want : kNoAllocBlocks);
+    k_dt_partial_noalloc<<<nblocks, kNoAllocThreads, 0, s>>>(dm, L, cs, v, layers, scratch);
+    k_dt_final_noalloc<<<1, 1024, 0, s>>>(scratch, nblocks, cfl, dt_old, deltat_max, out);
+  }
   if (cudaGetLastError() != cudaSuccess) return MHY_ERR_CUDA;
   return MHY_OK;
 }

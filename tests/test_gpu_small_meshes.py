@@ -1,0 +1,38 @@
+"""GPU: the kernel forms chosen by mesh size, at the sizes where the choice or
+its remainders change.  The allocation-free dt runs as one cluster up to 8192
+segments of 4 layers, else over segments of 4 or 8; the value is compared with
+its definition."""
+import numpy as np
+import pytest
+
+import mhy_b200
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (5, 3, 7), (100, 5, 5), (16, 16, 16), (17, 16, 16), (4097, 1, 1), (32, 32, 32),
+                               (32, 32, 33), (8193, 1, 3), (1, 1, 4099), (257, 3, 13), (600, 520, 9)])
+def test_allocation_free_dt_is_the_minimum_of_its_definition(n):
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = n
+    rng = np.random.default_rng(nx + ny + nz)
+    L, cs = rng.uniform(0.5, 2.0, (2, nz, ny, nx))
+    v = rng.normal(size=(3, nz + 1, ny + 1, nx + 1))
+    speed = np.sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2])
+    vmax = np.maximum.reduce([speed[dk:nz + dk, dj:ny + dj, di:nx + di] for dk in (0, 1) for dj in (0, 1) for di in (0, 1)])
+    want = (L / (cs + vmax)).min()
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (L, cs, v)]
+    out = torch.full((2,), -1.0, dtype=torch.float64, device="cuda")
+
+    def call():
+        torch.cuda.synchronize()
+        rc = mhy_b200.load().mhy_compute_hydro_dt_noalloc(nx, ny, nz, *(t.data_ptr() for t in dev), 0.3, 1e6, 1e6,
+                                                          out.data_ptr(), None)
+        torch.cuda.synchronize()
+        assert rc == 0
+        return out.cpu().numpy()
+
+    assert list(call()) == [want, 0.3 * want]
+    dev[0][-1, -1, -1] = -1.0                         # the last cell inverted
+    got = call()
+    assert np.isnan(got[0]) and got[1] == 0.0
