@@ -96,6 +96,8 @@ struct mhy_ctx {
   int phase = PH_SAVE;
   bool state_set = false, initialized = false;
   cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
+  double* dpf2 = nullptr;                        // small meshes: the second buffer of SweepFork
+  SweepFork fork{};                              // and its stream and events (made with the first graph)
   int kernels_per_cycle = 0;
   int lines[BK_COUNT] = {kLineWarps, kLineWarps, kLineWarps, kLineWarps, kLineWarps, kLineWarps, kLineWarps,
                          kLineWarps};                  // lines per block of the sweeps (the tuning)
@@ -300,6 +302,7 @@ int mhy_create(const mhy_mesh_desc* mesh, const mhy_options* opt, int device, mh
     if (rc == MHY_OK) rc = c->alloc(&c->pf, (size_t)C);
   }
   A_(&c->U[0], NV * C); A_(&c->U[1], NV * C);
+  if (C < kSmallMesh) A_(&c->dpf2, K * C);
   if (opt->conservation_energie_totale) { A_(&c->mfc, C); A_(&c->ecn, N); }
   if (K > 1) {
     EnvState& ev = c->env;
@@ -550,24 +553,24 @@ int launch_geometry(mhy_ctx* c) {
   else launch_lagrange_cells_env(c->args(), c->stream);
   return MHY_OK;
 }
-int launch_remap_(mhy_ctx* c, int sens, KernelMarks* m = nullptr) {
+int launch_remap_(mhy_ctx* c, int sens, KernelMarks* m = nullptr, SweepFork* fork = nullptr) {
   if (c->K == 1) {
     if (c->ph.csts) launch_csts_forward(c->args(), c->stream);   // PrepareRemap.cc:456, then the face velocities
-    launch_remap(c->args(), sens, c->stream, m);
+    launch_remap(c->args(), sens, c->stream, m, fork);
     if (c->ph.cons_ec) launch_cons_ec(c->args(), c->stream);   // after the last node sweep, before dt
   } else {
     if (c->ph.csts) launch_csts_forward(c->args(), c->stream);   // PrepareRemap.cc:456, then the face velocities
-    launch_remap_env(c->args(), sens, c->stream, m);
+    launch_remap_env(c->args(), sens, c->stream, m, fork);
     if (c->ph.cons_ec) launch_cons_ec_env(c->args(), c->stream);   // after the last node sweep, before dt
   }
   return MHY_OK;
 }
 int launch_delta_t_(mhy_ctx* c) { launch_delta_t(c->args(), c->stream); return MHY_OK; }
 
-int launch_cycle(mhy_ctx* c, int sens) {
+int launch_cycle(mhy_ctx* c, int sens, SweepFork* fork) {
   launch_velocity(c);
   launch_geometry(c);
-  launch_remap_(c, sens);
+  launch_remap_(c, sens, nullptr, fork);
   launch_delta_t_(c);
   return MHY_OK;
 }
@@ -575,9 +578,16 @@ int launch_cycle(mhy_ctx* c, int sens) {
 // The cycle graph of direction rotation s (captured once).
 int cycle_graph(mhy_ctx* c, int s) {
   if (c->graph[s]) return MHY_OK;
+  if (c->dpf2 && !c->fork.side) {
+    c->fork.dpf[0] = c->dpf;
+    c->fork.dpf[1] = c->dpf2;
+    for (cudaEvent_t& e : c->fork.ev)
+      if (!e) MHY_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    MHY_CUDA(cudaStreamCreateWithFlags(&c->fork.side, cudaStreamNonBlocking));
+  }
   cudaGraph_t g = nullptr;
   MHY_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  launch_cycle(c, s);
+  launch_cycle(c, s, c->dpf2 ? &c->fork : nullptr);
   cudaError_t le = cudaGetLastError();
   cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
   if (le != cudaSuccess || ee != cudaSuccess)
@@ -1883,6 +1893,8 @@ void mhy_destroy(mhy_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (int s = 0; s < 3; ++s) if (c->graph[s]) cudaGraphExecDestroy(c->graph[s]);
   for (void* p_ : c->allocs) cudaFree(p_);
+  for (cudaEvent_t e : c->fork.ev) if (e) cudaEventDestroy(e);
+  if (c->fork.side) cudaStreamDestroy(c->fork.side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

@@ -53,10 +53,38 @@ __device__ __forceinline__ D3 node_force(const Dims& dm, int i, int j, int k, co
   return F;
 }
 
+// The same sum with every load issued before the first addition: the loads of
+// the form above follow one another in groups, cell by cell, which costs little
+// where many warps are in flight and eight round trips where few are.
+template <typename CQ>
+__device__ __forceinline__ D3 node_force_gathered(const Dims& dm, int i, int j, int k, const double* __restrict__ p,
+                                                  const double* __restrict__ q, const CQ* __restrict__ cqs) {
+  const int loc[2][2][2] = {{{0, 4}, {3, 7}}, {{1, 5}, {2, 6}}};
+  double pc[8], qc[8];
+  CQ w[8][3];
+  bool in[8];
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    const int di = ~a & 1, dj = ~(a >> 1) & 1, dk = ~(a >> 2) & 1, ci = i - di, cj = j - dj, ck = k - dk;
+    in[a] = !(ci < 0 || cj < 0 || ck < 0 || ci >= dm.nx || cj >= dm.ny || ck >= dm.nz);
+    const long long c = in[a] ? dm.cid(ci, cj, ck) : 0;
+    const int l = loc[di][dj][dk];
+    pc[a] = p[c];
+    qc[a] = q[c];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) w[a][e] = cqs[(l * 3 + e) * dm.C + c];
+  }
+  D3 F = d3(0, 0, 0);
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+    if (in[a]) F = F + (pc[a] + qc[a]) * d3((double)w[a][0], (double)w[a][1], (double)w[a][2]);
+  return F;
+}
+
 // vnb (schema-csts only, else null): v_n taken back from n to n-1/2 with
 // the same force first, updateVelocityBackward (MahycoModule.cc:693, 743-781),
 // and kept for the energy and the remap face velocities.
-template <typename CQ>
+template <typename CQ, bool GATHERED = false>
 __device__ __forceinline__ void k_cyc_lagrange_nodes_body(Dims dm, const Scalars* __restrict__ S,
     const double* __restrict__ p, const double* __restrict__ q, const CQ* __restrict__ cqs,
     const double* __restrict__ nm, const double* __restrict__ v, const uint16_t* __restrict__ bcmask, BCTable bct,
@@ -66,7 +94,9 @@ __device__ __forceinline__ void k_cyc_lagrange_nodes_body(Dims dm, const Scalars
   if (!block_item(dm.nx + 1, dm.ny + 1, dm.nz + 1, bx_, by_, bz_, i, j, k)) return;
   const long long n = dm.nid(i, j, k);
   const double dtv = 0.5 * (S->old_dt + S->dt);
-  const D3 F = node_force<CQ>(dm, i, j, k, p, q, cqs);
+  D3 F;
+  if constexpr (GATHERED) F = node_force_gathered<CQ>(dm, i, j, k, p, q, cqs);
+  else F = node_force<CQ>(dm, i, j, k, p, q, cqs);
   const double s = dtv / nm[n];
   D3 vb = d3(v[n], v[dm.N + n], v[2 * dm.N + n]);
   if (vnb) {
@@ -86,12 +116,12 @@ __device__ __forceinline__ void k_cyc_lagrange_nodes_body(Dims dm, const Scalars
   vh[n] = u.x; vh[dm.N + n] = u.y; vh[2 * dm.N + n] = u.z;
 }
 
-template <typename CQ>
+template <typename CQ, bool GATHERED>
 __global__ void __launch_bounds__(128) k_cyc_lagrange_nodes(Dims dm, const Scalars* __restrict__ S,
     const double* __restrict__ p, const double* __restrict__ q, const CQ* __restrict__ cqs,
     const double* __restrict__ nm, const double* __restrict__ v, const uint16_t* __restrict__ bcmask, BCTable bct,
     double* __restrict__ vh, double* __restrict__ vnb) {
-  k_cyc_lagrange_nodes_body<CQ>(dm, S, p, q, cqs, nm, v, bcmask, bct, vh, vnb, blockIdx.x, -1, 0);
+  k_cyc_lagrange_nodes_body<CQ, GATHERED>(dm, S, p, q, cqs, nm, v, bcmask, bct, vh, vnb, blockIdx.x, -1, 0);
 }
 
 // schema-csts, updateVelocityForward (PrepareRemap.cc:456, MahycoModule.cc:
@@ -489,12 +519,15 @@ static void sweep_cells_d(const CycleArgs& a, bool last, const double* Uin, doub
 // most of a second block idle).
 void launch_lagrange_nodes(const CycleArgs& a, cudaStream_t s) {
   const unsigned nbn = (unsigned)((a.dm.N + 127) / 128);
-  if (a.ph.precision)
-    k_cyc_lagrange_nodes<float><<<nbn, 128, 0, s>>>(a.dm, a.S, a.st.p, a.st.q, a.cqs32, a.nm, a.v, a.bcmask, a.bct, a.vh,
-                                                    nullptr);
-  else
-    k_cyc_lagrange_nodes<double><<<nbn, 128, 0, s>>>(a.dm, a.S, a.st.p, a.st.q, a.cqs, a.nm, a.v, a.bcmask, a.bct, a.vh,
-                                                     a.ph.csts ? a.vnb : nullptr);
+  const bool few = a.dm.C < kSmallMesh;
+  if (a.ph.precision) {
+    auto kern = few ? k_cyc_lagrange_nodes<float, true> : k_cyc_lagrange_nodes<float, false>;
+    kern<<<nbn, 128, 0, s>>>(a.dm, a.S, a.st.p, a.st.q, a.cqs32, a.nm, a.v, a.bcmask, a.bct, a.vh, nullptr);
+  } else {
+    auto kern = few ? k_cyc_lagrange_nodes<double, true> : k_cyc_lagrange_nodes<double, false>;
+    kern<<<nbn, 128, 0, s>>>(a.dm, a.S, a.st.p, a.st.q, a.cqs, a.nm, a.v, a.bcmask, a.bct, a.vh,
+                             a.ph.csts ? a.vnb : nullptr);
+  }
 }
 
 void launch_csts_forward(const CycleArgs& a, cudaStream_t s) {
@@ -608,10 +641,11 @@ __global__ void __launch_bounds__(128) k_o3_faces(Dims dm, const Scalars* __rest
 }
 
 template <typename R>
-static void remap_impl(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m) {
+static void remap_impl(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m, SweepFork* fork) {
   int prev = 0;
   CycleArgs a = a0;
   for (int it = 0; it < 3; ++it) {
+    if (fork) fork->begin_cells(a, it, s);
     const int d = (it + sens) % 3;
     const bool first = it == 0, last = it == 2;
     a.ph.pb_first = first;
@@ -630,7 +664,7 @@ static void remap_impl(const CycleArgs& a0, int sens, cudaStream_t s, KernelMark
     else if (d == 1) sweep_cells_d<1, R>(a, last, uin, uout, s);
     else sweep_cells_d<2, R>(a, last, uin, uout, s);
     mark(m, BK_CELLS_X + d, s);
-    sweep_nodes<1, R>(a, d, first, last, prev, udin, udout, s);
+    sweep_nodes<1, R>(a, d, first, last, prev, udin, udout, fork ? fork->nodes_stream(it, s) : s);
     mark(m, BK_NODES_X + d, s);
     prev |= 1 << d;
   }
@@ -673,17 +707,17 @@ void launch_cons_ec(const CycleArgs& a, cudaStream_t s) {
   k_cons_ec<<<nbc, 128, 0, s>>>(a.dm, a.ph, a.ecn, a.st.mf, a.st.rho, a.st.e, a.st.p, a.st.cs, linear);
 }
 
-void launch_remap(const CycleArgs& a, int sens, cudaStream_t s, KernelMarks* m) {
-  if (a.ph.precision) { remap_impl<float>(a, sens, s, m); return; }
+void launch_remap(const CycleArgs& a, int sens, cudaStream_t s, KernelMarks* m, SweepFork* fork) {
+  if (a.ph.precision) { remap_impl<float>(a, sens, s, m, fork); return; }
   if (a.ph.csts) {
     // schema-csts: the remap starts from the forward velocity (U_dual,
     // Phi_dual, PrepareRemap.cc:411-433) on the Lagrangian coordinates
     CycleArgs b = a;
     b.vh = a.vf;
-    remap_impl<double>(b, sens, s, m);
+    remap_impl<double>(b, sens, s, m, fork);
     return;
   }
-  remap_impl<double>(a, sens, s, m);
+  remap_impl<double>(a, sens, s, m, fork);
 }
 
 void launch_delta_t(const CycleArgs& a, cudaStream_t s) {

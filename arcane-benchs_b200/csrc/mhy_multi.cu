@@ -982,9 +982,11 @@ static void env_cells(const CycleArgs& a, int d, const double* Uin, double* Uout
 
 // R: evaluation type of the sweeps (double, or float in the mixed form).
 template <int K, typename R>
-static void remap_env(const CycleArgs& a, int sens, cudaStream_t s, KernelMarks* m) {
+static void remap_env(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m, SweepFork* fork) {
   int prev = 0;
+  CycleArgs a = a0;
   for (int it = 0; it < 3; ++it) {
+    if (fork) fork->begin_cells(a, it, s);
     const int d = (it + sens) % 3;
     const bool first = it == 0, last = it == 2;
     const double* uin = a.U[it & 1];
@@ -1005,7 +1007,7 @@ static void remap_env(const CycleArgs& a, int sens, cudaStream_t s, KernelMarks*
       k_env_finalize_cells<K><<<nb, 256, 0, s>>>(a.dm, a.S, a.ph, a.env, uout, a.st, a.fd);
     }
     mark(m, BK_CELLS_X + d, s);
-    sweep_nodes<K, R>(a, d, first, last, prev, udin, udout, s);
+    sweep_nodes<K, R>(a, d, first, last, prev, udin, udout, fork ? fork->nodes_stream(it, s) : s);
     mark(m, BK_NODES_X + d, s);
     prev |= 1 << d;
   }
@@ -1047,19 +1049,19 @@ void launch_lagrange_cells_env(const CycleArgs& a, cudaStream_t s) {
   else launch_cells<4>(a, s);
 }
 
-void launch_remap_env(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m) {
+void launch_remap_env(const CycleArgs& a0, int sens, cudaStream_t s, KernelMarks* m, SweepFork* fork) {
   // schema-csts: the remap starts from the forward velocity (U_dual,
   // Phi_dual, PrepareRemap.cc:411-433) on the Lagrangian coordinates
   CycleArgs a = a0;
   if (a.ph.csts) a.vh = a.vf;
   if (a.ph.precision) {
-    if (a.K == 2) remap_env<2, float>(a, sens, s, m);
-    else if (a.K == 3) remap_env<3, float>(a, sens, s, m);
-    else remap_env<4, float>(a, sens, s, m);
+    if (a.K == 2) remap_env<2, float>(a, sens, s, m, fork);
+    else if (a.K == 3) remap_env<3, float>(a, sens, s, m, fork);
+    else remap_env<4, float>(a, sens, s, m, fork);
   } else {
-    if (a.K == 2) remap_env<2, double>(a, sens, s, m);
-    else if (a.K == 3) remap_env<3, double>(a, sens, s, m);
-    else remap_env<4, double>(a, sens, s, m);
+    if (a.K == 2) remap_env<2, double>(a, sens, s, m, fork);
+    else if (a.K == 3) remap_env<3, double>(a, sens, s, m, fork);
+    else remap_env<4, double>(a, sens, s, m, fork);
   }
 }
 

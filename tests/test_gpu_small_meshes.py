@@ -1,13 +1,40 @@
 """GPU: the kernel forms chosen by mesh size, at the sizes where the choice or
-its remainders change.  The allocation-free dt runs as one cluster up to 8192
-segments of 4 layers, else over segments of 4 or 8; the value is compared with
-its definition."""
+its remainders change.  The cycle graph below 131072 cells runs node and cell
+sweeps side by side; a batch, which never does, must give the same bits.  The
+allocation-free dt runs as one cluster up to 8192 segments of 4 layers, else over
+segments of 4 or 8; the value is compared with its definition."""
 import numpy as np
 import pytest
 
 import mhy_b200
+from mhy_b200 import Batch, Context, gen
 
 pytestmark = pytest.mark.gpu
+
+FIELDS = ("density", "internal_energy", "pressure", "velocity", "node_mass")
+
+
+@pytest.mark.parametrize("options", [{}, {"precision": 1}, {"ordre_projection": 3}, {"projection_limiteur_id": 4}])
+@pytest.mark.parametrize("K", [1, 2])
+def test_graph_of_a_small_mesh_equals_a_batch(K, options):
+    o = gen.Options(**options)
+    sizes = ((3, 3, 3), (33, 9, 4), (64, 64, 31), (64, 64, 32))      # the last one is not small
+    if K == 1:
+        cases = [gen.sod(*n, lx=n[0] * 0.01, ly=n[1] * 0.01, lz=n[2] * 0.01, jitter=0.02, seed=i, options=o)
+                 for i, n in enumerate(sizes)]
+    else:
+        cases = [gen.two_material(*n, seed=i, options=o) for i, n in enumerate(sizes)]
+    b = Batch(cases, device=0)
+    b.step(12)
+    b.synchronize()
+    for i, c in enumerate(cases):
+        g = Context(c, device=0)
+        g.step(12)                                    # each rotation's graph four times
+        g.synchronize()
+        for f in FIELDS:
+            assert np.array_equal(b.field(i, f), g.field(f)), (i, f)
+        assert b.dt(i) == g.dt(), i
+        g.close()
 
 
 @pytest.mark.parametrize("n", [(1, 1, 1), (5, 3, 7), (100, 5, 5), (16, 16, 16), (17, 16, 16), (4097, 1, 1), (32, 32, 32),
