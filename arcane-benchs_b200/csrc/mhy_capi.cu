@@ -609,6 +609,13 @@ int flush(mhy_ctx* c) {
   return MHY_OK;
 }
 
+// The device scalars behind everything queued on the context's stream: one
+// ordered copy and one wait.
+cudaError_t read_scalars(mhy_ctx* c, Scalars& h) {
+  const cudaError_t e = cudaMemcpyAsync(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+}
+
 #define MHY_FLUSH(c)                  \
   do {                                \
     const int frc_ = flush(c);        \
@@ -700,9 +707,8 @@ int mhy_synchronize(mhy_ctx* c) {
   if (!c) return fail(MHY_ERR_ARG, "null context");
   DeviceScope on_dev(c->device);
   MHY_FLUSH(c);
-  MHY_CUDA(cudaStreamSynchronize(c->stream));
   Scalars h{};
-  MHY_CUDA(cudaMemcpy(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost));
+  MHY_CUDA(read_scalars(c, h));
   if (h.status & MHY_STATUS_DT_MIN) return fail(MHY_ERR_DT_MIN, "dt fell below deltat-min");
   if (h.status & (MHY_STATUS_NAN_DT | MHY_STATUS_ZERO_MASS)) return fail(MHY_ERR_NUMERIC, "numeric status raised on the device");
   return MHY_OK;
@@ -1577,9 +1583,8 @@ int mhy_checkpoint_save(mhy_ctx* c, void* dst, size_t bytes) {
   std::vector<int64_t> off;
   const size_t need = ckpt_layout(f, off);
   if (bytes < need) return fail(MHY_ERR_ARG, "destination too small (mhy_checkpoint_size)");
-  MHY_CUDA(cudaStreamSynchronize(c->stream));
   Scalars h{};
-  MHY_CUDA(cudaMemcpy(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost));
+  MHY_CUDA(read_scalars(c, h));
   char* base = static_cast<char*>(dst);
   std::memset(base, 0, sizeof(CkptHeader) + f.size() * sizeof(CkptField));
   CkptHeader hd{};
@@ -1716,8 +1721,7 @@ int mhy_get_dt(mhy_ctx* c, double* dt, double* dt_old) {
   DeviceScope on_dev(c->device);
   MHY_FLUSH(c);
   Scalars h{};
-  MHY_CUDA(cudaStreamSynchronize(c->stream));
-  MHY_CUDA(cudaMemcpy(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost));
+  MHY_CUDA(read_scalars(c, h));
   if (dt) *dt = h.dt;
   if (dt_old) *dt_old = h.old_dt;
   return MHY_OK;
@@ -1728,8 +1732,7 @@ int mhy_get_time(mhy_ctx* c, double* time, int64_t* iteration) {
   DeviceScope on_dev(c->device);
   MHY_FLUSH(c);
   Scalars h{};
-  MHY_CUDA(cudaStreamSynchronize(c->stream));
-  MHY_CUDA(cudaMemcpy(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost));
+  MHY_CUDA(read_scalars(c, h));
   if (time) *time = h.time;
   if (iteration) *iteration = h.iteration;
   return MHY_OK;
@@ -1740,8 +1743,7 @@ int mhy_get_status(mhy_ctx* c, uint32_t* flags) {
   DeviceScope on_dev(c->device);
   MHY_FLUSH(c);
   Scalars h{};
-  MHY_CUDA(cudaStreamSynchronize(c->stream));
-  MHY_CUDA(cudaMemcpy(&h, c->S, sizeof(h), cudaMemcpyDeviceToHost));
+  MHY_CUDA(read_scalars(c, h));
   *flags = h.status;
   return MHY_OK;
 }
