@@ -756,7 +756,7 @@ std::vector<int4> build_work(const std::vector<mhy_ctx*>& inst, int kind, int or
       batch_column_shape(inst[i]->dm, gx, gy, strip);
       gz = 1;
     } else {
-      batch_work_shape(inst[i]->dm, kind, lines, march, gx, gy, gz);
+      batch_work_shape(inst[i]->dm, inst[i]->K, kind, lines, march, gx, gy, gz);
     }
     if (gy < 0) {                               // linear chunks of consecutive items
       for (int x = 0; x < gx; ++x) per[i].push_back(make_int4(i, x, -1, 0));

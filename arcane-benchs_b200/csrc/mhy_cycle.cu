@@ -188,18 +188,17 @@ __global__ void __launch_bounds__(128) k_csts_face_u(Dims dm, const double* __re
 template <bool LAST, typename R, bool O3, bool GL, bool PB, bool SP>
 __device__ __forceinline__ void cells_x_line(const Dims& dm, const Scalars* __restrict__ S, const Phys& ph,
     const FaceData& fd, const double* __restrict__ n0, const double* __restrict__ xcs, const double* __restrict__ ofn,
-    const double* __restrict__ Uin, const double* __restrict__ Ve, int bx_, int by_, int bz_, double* out,
+    const double* __restrict__ Uin, const double* __restrict__ Ve, int bx_, double* out,
     unsigned* oor) {
   const int lane = threadIdx.x & 31;
-  const int j = by_ * kLineWarps + (threadIdx.x >> 5), k = bz_;
   const int nd = dm.nx, C = (int)dm.C, F = (int)dm.F;
-  const int s = bx_ * kLineUpd - 2 + lane;      // position of this lane's cell along x
-  const bool valid = s >= 0 && s < nd;
-  const bool inner = s >= 1 && s <= nd - 1;            // this lane's low face is an inner face
-  const bool infr = s + 1 <= nd - 1;
+  const RowPos rp = row_pos(bx_, nd, dm.ny, C);
+  const int s = rp.s, c = rp.id;                // s: position of this lane's cell along x
+  const bool valid = rp.valid;
+  const bool inner = valid && s >= 1;                  // this lane's low face is an inner face
+  const bool infr = valid && s + 1 <= nd - 1;
   const bool upd = valid && lane >= 2 && lane < 2 + kLineUpd;
-  const int c = valid ? s + dm.nx * (j + dm.ny * k) : 0;
-  const int t = inner ? s + (dm.nx + 1) * (j + dm.ny * k) : 0;   // x faces come first: t is also the face id
+  const int t = inner ? c + rp.j + dm.ny * rp.k : 0;   // a row of faces is one longer; x faces come first
   CellIn in;
   in.U[0] = in.U[1] = in.U[2] = in.U[3] = 0.; in.xc[0] = in.xc[1] = in.xc[2] = 0.;
   in.db = in.df = in.u = in.A = 0.; in.n[0] = in.n[1] = in.n[2] = 0.; in.ob = in.of = in.vol = 0.; in.h = 0.;
@@ -232,9 +231,9 @@ __device__ __forceinline__ void cells_x_line(const Dims& dm, const Scalars* __re
 template <bool LAST, typename R, bool O3, bool GL, bool PB>
 __device__ __noinline__ LineOut<LAST ? kCellOutLast : kCellOutMid> cells_x_line_exact(Dims dm, const Scalars* S,
     Phys ph, FaceData fd, const double* n0, const double* xcs, const double* ofn, const double* Uin, const double* Ve,
-    int bx_, int by_, int bz_) {
+    int bx_) {
   LineOut<LAST ? kCellOutLast : kCellOutMid> o;
-  cells_x_line<LAST, R, O3, GL, PB, false>(dm, S, ph, fd, n0, xcs, ofn, Uin, Ve, bx_, by_, bz_, o.v, nullptr);
+  cells_x_line<LAST, R, O3, GL, PB, false>(dm, S, ph, fd, n0, xcs, ofn, Uin, Ve, bx_, o.v, nullptr);
   return o;
 }
 
@@ -243,28 +242,24 @@ __device__ __forceinline__ void k_cyc_sweep_cells_x_body(Dims dm, const Scalars*
     Phys ph, FaceData fd, const double* __restrict__ n0, const double* __restrict__ xcs,
     const double* __restrict__ ofn, const double* __restrict__ Uin, double* __restrict__ Uout,
     double* __restrict__ dpf, CellState st,
-    int bx_, int by_, int bz_) {
+    int bx_) {
   constexpr int NO = LAST ? kCellOutLast : kCellOutMid;
   const int lane = threadIdx.x & 31;
-  const int j = by_ * kLineWarps + (threadIdx.x >> 5), k = bz_;
-  if (j >= dm.ny) return;                              // whole warp leaves together
+  if (row_first(bx_) >= (int)dm.C) return;             // whole warp leaves together
   double out[NO];
   if constexpr (sizeof(R) == 8 && !PB) {
     unsigned oor = 0u;
-    cells_x_line<LAST, R, O3, GL, PB, true>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_, by_, bz_, out, &oor);
+    cells_x_line<LAST, R, O3, GL, PB, true>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_, out, &oor);
     if (__any_sync(0xffffffffu, oor != 0u)) {
-      const auto o = cells_x_line_exact<LAST, R, O3, GL, PB>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_, by_, bz_);
+      const auto o = cells_x_line_exact<LAST, R, O3, GL, PB>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_);
 #pragma unroll
       for (int a = 0; a < NO; ++a) out[a] = o.v[a];
     }
   } else {
-    cells_x_line<LAST, R, O3, GL, PB, false>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_, by_, bz_, out, nullptr);
+    cells_x_line<LAST, R, O3, GL, PB, false>(dm, S, ph, fd, n0, xcs, ofn, Uin, st.Ve, bx_, out, nullptr);
   }
-  const int nd = dm.nx, C = (int)dm.C;
-  const int s = bx_ * kLineUpd - 2 + lane;
-  const bool upd = s >= 0 && s < nd && lane >= 2 && lane < 2 + kLineUpd;
-  const int c = s + dm.nx * (j + dm.ny * k);
-  if (!upd) return;
+  const int C = (int)dm.C, c = row_first(bx_) - 2 + lane;
+  if (c >= C || lane < 2 || lane >= 2 + kLineUpd) return;
   if (!LAST) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) Uout[v * C + c] = out[v];
@@ -281,8 +276,7 @@ __global__ void __launch_bounds__(32 * kLineWarps, kLineMinBlocks) k_cyc_sweep_c
     Phys ph, FaceData fd, const double* __restrict__ n0, const double* __restrict__ xcs,
     const double* __restrict__ ofn, const double* __restrict__ Uin, double* __restrict__ Uout,
     double* __restrict__ dpf, CellState st) {
-  k_cyc_sweep_cells_x_body<LAST, R, O3, GL, PB>(dm, S, ph, fd, n0, xcs, ofn, Uin, Uout, dpf, st, blockIdx.x, blockIdx.y,
-                                        blockIdx.z);
+  k_cyc_sweep_cells_x_body<LAST, R, O3, GL, PB>(dm, S, ph, fd, n0, xcs, ofn, Uin, Uout, dpf, st, blockIdx.x);
 }
 
 // Cell sweep along y (D = 1) or z (D = 2), staged through shared memory.
@@ -486,10 +480,9 @@ static void sweep_cells_t(const CycleArgs& a, const double* Uin, double* Uout, c
 template <int D, typename R>
 static void sweep_cells_d(const CycleArgs& a, bool last, const double* Uin, double* Uout, cudaStream_t s) {
   const Dims& dm = a.dm;
-  const int nseg = (dm.ncd(D) + kLineUpd - 1) / kLineUpd;
   const int T = 32 * kLineWarps;
   if constexpr (D == 0) {
-    const dim3 g(nseg, (dm.ny + kLineWarps - 1) / kLineWarps, dm.nz);
+    const int g = row_chunks(dm.C);
     const bool o3 = sizeof(R) == 8 && a.ph.ordre_projection == 3;
     const bool gl = sizeof(R) == 8 && a.ph.ordre_projection > 1 && a.ph.lim_cell >= 3;
     if constexpr (sizeof(R) == 8) {
@@ -733,7 +726,7 @@ void launch_delta_t(const CycleArgs& a, cudaStream_t s) {
 // work item with a barrier, since the previous item's last reads of the tile
 // may still be in flight in other warps.
 
-void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, int& gy, int& gz) {
+void batch_work_shape(const Dims& dm, int K, int kind, int lines, bool march, int& gx, int& gy, int& gz) {
   const int nx = dm.nx, ny = dm.ny, nz = dm.nz;
   auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
   const int W = lines;                            // lines per block of the y/z sweeps
@@ -750,10 +743,13 @@ void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, 
       if (nx % 128) { gx = (int)cdiv((int)dm.C, 128); gy = -1; gz = 1; }        // linear chunks
       else { gx = nx / 128; gy = ny; gz = nz; }
       break;
-    case BK_CELLS_X: gx = cdiv(nx, kLineUpd); gy = cdiv(ny, kLineWarps); gz = nz; break;
+    case BK_CELLS_X:
+      if (K == 1) { gx = row_chunks(dm.C); gy = gz = 1; }                      // chunks of the rows' sequence
+      else { gx = cdiv(nx, kLineUpd); gy = cdiv(ny, kLineWarps); gz = nz; }
+      break;
     case BK_CELLS_Y: gx = cdiv(nx, W); gy = cdiv(ny, kLineUpd); gz = nz; break;
     case BK_CELLS_Z: gx = cdiv(nx, W); gy = cdiv(nz, kLineUpd); gz = ny; break;
-    case BK_NODES_X: gx = cdiv(nx + 1, kLineUpd); gy = cdiv(ny + 1, kLineWarps); gz = nz + 1; break;
+    case BK_NODES_X: gx = row_chunks(dm.N); gy = gz = 1; break;
     case BK_NODES_Y: gx = cdiv(nx + 1, W); gy = cdiv(ny + 1, kLineUpd); gz = nz + 1; break;
     default: gx = cdiv(nx + 1, W); gy = cdiv(nz + 1, kLineUpd); gz = ny + 1; break;
   }
@@ -805,10 +801,10 @@ __global__ void __launch_bounds__(32 * kLineWarps, kLineMinBlocks) k_bat_sweep_c
       Phys ph = a.ph;
       ph.pb_first = it == 0;
       k_cyc_sweep_cells_x_body<LAST, R, O3, GL, PB>(a.dm, a.S, ph, a.fd, a.n0, a.xc, a.ofn, a.U[it & 1],
-                                                a.U[(it + 1) & 1], a.dpf, a.st, t.y, t.z, t.w);
+                                                a.U[(it + 1) & 1], a.dpf, a.st, t.y);
     } else {
       k_cyc_sweep_cells_x_body<LAST, R, O3, GL, PB>(a.dm, a.S, a.ph, a.fd, a.n0, a.xc, a.ofn, a.U[it & 1],
-                                                a.U[(it + 1) & 1], a.dpf, a.st, t.y, t.z, t.w);
+                                                a.U[(it + 1) & 1], a.dpf, a.st, t.y);
     }
   }
 }
@@ -853,7 +849,7 @@ __global__ void __launch_bounds__(32 * kLineWarps, kLineMinBlocks) k_bat_sweep_n
     // schema-csts: the forward velocity on the Lagrangian coordinates (xl is null otherwise)
     k_cyc_sweep_nodes_x_body<FIRST, LAST, 1, R, GL>(a.dm, a.S, a.ph, prev, a.x0, a.xl, a.ph.csts ? a.vf : a.vh, a.nm,
                                                  a.ud[(it + 1) & 1], a.ud[it & 1], a.dpf, a.Gd, a.st.mass, a.v, a.nm,
-                                                 a.vnorm, t.y, t.z, t.w, a.ecn);
+                                                 a.vnorm, t.y, a.ecn);
   }
 }
 

@@ -217,7 +217,7 @@ struct KernelMarks {
   int n;
 };
 // Blocks of one instance's grid for a kernel kind; march: its y/z sweep marches (BatchPlan::march).
-void batch_work_shape(const Dims& dm, int kind, int lines, bool march, int& gx, int& gy, int& gz);
+void batch_work_shape(const Dims& dm, int K, int kind, int lines, bool march, int& gx, int& gy, int& gz);
 bool batch_marches(const CycleArgs& a, int kind, long long nodes);
 void batch_column_shape(const Dims& dm, int& blocks, int& segments, int& strip);
 // Dynamic shared memory above the default 48 KB needs an opt-in per kernel and device.

@@ -25,6 +25,38 @@ namespace mhy {
 // element offset fits).
 
 constexpr int kLineUpd = 28;    // items updated per warp (32 lanes, 2 halo lanes on each side)
+
+// The x sweeps (but the cells of several environments) take the cells (nodes)
+// of the whole mesh as one sequence, row
+// after row: warp w of chunk b updates items 28 (8 b + w) .. + 27 and its lanes
+// hold two more on each side, whatever row they lie in.  What a lane reads from
+// a neighbour of another row is masked as at a row's end (its position in the
+// row decides, not the lane).  Rows of their own segments left lanes idle: 33
+// nodes took two warps, 129 took five.  Measured on B200, rows -> sequence:
+// FP64 batch of 32^3..96^3, cells 479 -> 389 and last 870 -> 680 us, nodes 655 ->
+// 536, 699 -> 556 and last 878 -> 751 us; Sedov 128^3, cells 70 -> 65 and last
+// 96 -> 89 us, nodes 75 to 109 us either way.  The cells of several environments
+// keep their rows: at 128 registers the positions spill (two gases 256x128x128,
+// 264 -> 316 us).
+struct RowPos {
+  int s, j, k, id;                // position along x, row, layer; the item's number
+  bool valid;
+};
+__device__ __forceinline__ int row_first(int chunk) {              // the first item a warp updates
+  return (chunk * kLineWarps + (int)(threadIdx.x >> 5)) * kLineUpd;
+}
+__device__ __forceinline__ RowPos row_pos(int chunk, int n, int rows, int total) {   // n items a row
+  RowPos p;
+  p.id = row_first(chunk) - 2 + (int)(threadIdx.x & 31);
+  p.valid = p.id >= 0 && p.id < total;
+  if (!p.valid) p.id = 0;
+  const unsigned row = (unsigned)p.id / (unsigned)n;
+  p.s = p.id - (int)row * n;
+  p.k = (int)(row / (unsigned)rows);
+  p.j = (int)row - p.k * rows;
+  return p;
+}
+inline int row_chunks(long long total) { return (int)((total + kLineUpd * kLineWarps - 1) / (kLineUpd * kLineWarps)); }
 // The sweeps are latency bound (long dependent chains of divisions and
 // shuffles per lane); 4 resident blocks (32 warps, 64 registers, a few bytes
 // of spill) per SM run them 15 % faster than the 2-3 blocks the compiler's
@@ -566,7 +598,8 @@ constexpr int kNodeOutLast = 6;   // the last sweep adds the node's conservation
 template <int D, bool FIRST, bool LAST, typename R = double, bool GL = false, bool SP = false>
 __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid, bool inner, bool updated,
                                           bool upd, const NodeIn& in, R G[3], double* out, bool xabs = false,
-                                          bool bb_ok = true, bool ff_ok = true, unsigned* oor = nullptr) {
+                                          bool bb_ok = true, bool ff_ok = true, unsigned* oor = nullptr,
+                                          bool starts = false) {
   const R order2 = (R)(ph.ordre_projection - 1);
   const int lim = ph.ordre_projection > 1 ? ph.limiteur_id : -1;
   const bool grad_on = ph.ordre_projection > 1;
@@ -601,13 +634,14 @@ __device__ __forceinline__ void node_line(const Phys& ph, double dt, bool valid,
     // front difference quotient of this node = back difference quotient of the next
     R gf[3], gb[3];
     // speculative quotients count only where they are used: a valid node
-    // whose next node is valid and in this warp (the last lane divides by 0)
+    // whose next node is valid, of its line (starts: the first of a line) and
+    // in this warp (the last lane divides by 0)
     unsigned gfo = 0u;
     const R hf = (R)(xp - x), rf = rc<R, SP>(hf, &gfo);
 #pragma unroll
     for (int c = 0; c < 3; ++c) gf[c] = dv<R, SP>(Pp[c] - P[c], hf, rf, &gfo);
     if constexpr (SP) {
-      const int next_valid = __shfl_down_sync(full, valid ? 1 : 0, 1);   // every lane takes part
+      const int next_valid = __shfl_down_sync(full, valid && !starts ? 1 : 0, 1);   // every lane takes part
       if (valid && (threadIdx.x & 31) < 31 && next_valid != 0) *oor |= gfo;
     }
 #pragma unroll
@@ -696,17 +730,16 @@ template <bool FIRST, bool LAST, int K, typename R, bool GL, bool SP>
 __device__ __forceinline__ void nodes_x_line(const Dims& dm, const Scalars* __restrict__ S, const Phys& ph,
     int prev_inner, const double* __restrict__ x0, const double* __restrict__ xl, const double* __restrict__ vh,
     const double* __restrict__ nm_in, const double* __restrict__ udin, const double* __restrict__ dpf,
-    const double* __restrict__ Gd, const double* __restrict__ mass, int bx_, int by_, int bz_, R G[3], double* out,
+    const double* __restrict__ Gd, const double* __restrict__ mass, int bx_, R G[3], double* out,
     unsigned* oor) {
   const int lane = threadIdx.x & 31;
-  const int j = by_ * kLineWarps + (threadIdx.x >> 5), k = bz_;
   const int nx = dm.nx, ny = dm.ny, nz = dm.nz, N = (int)dm.N;
-  const int m = bx_ * kLineUpd - 2 + lane;      // position of this lane's node along x
-  const bool valid = m >= 0 && m <= nx;
-  const bool inner = m >= 1 && m <= nx - 1;
+  const RowPos rp = row_pos(bx_, nx + 1, ny + 1, N);
+  const int m = rp.s, j = rp.j, k = rp.k, n = rp.id;   // m: position of this lane's node along x
+  const bool valid = rp.valid;
+  const bool inner = valid && m >= 1 && m <= nx - 1;
   const bool upd = valid && lane >= 2 && lane < 2 + kLineUpd;
-  const int idx[3] = {valid ? m : 0, j, k};
-  const int n = idx[0] + (nx + 1) * (j + (ny + 1) * k);
+  const int idx[3] = {m, j, k};
   const bool updated = node_updated(dm, 0, prev_inner, idx);
   const bool grad_on = ph.ordre_projection > 1;
   NodeIn in;
@@ -763,17 +796,16 @@ __device__ __forceinline__ void nodes_x_line(const Dims& dm, const Scalars* __re
     }
   }
   node_line<0, FIRST, LAST, R, GL, SP>(ph, S->dt, valid, inner, updated, upd, in, G, out, xl != nullptr, m >= 2,
-                                       m + 2 <= nx, oor);
+                                       m + 2 <= nx, oor, m == 0);
 }
 
 template <bool FIRST, bool LAST, int K, typename R, bool GL>
 __device__ __noinline__ NodeLineOut nodes_x_line_exact(Dims dm, const Scalars* S, Phys ph, int prev_inner,
     const double* x0, const double* xl, const double* vh, const double* nm_in, const double* udin, const double* dpf,
-    const double* Gd, const double* mass, int bx_, int by_, int bz_) {
+    const double* Gd, const double* mass, int bx_) {
   NodeLineOut o;
   R G[3];
-  nodes_x_line<FIRST, LAST, K, R, GL, false>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, by_,
-                                             bz_, G, o.v, nullptr);
+  nodes_x_line<FIRST, LAST, K, R, GL, false>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, G, o.v, nullptr);
   o.g[0] = (double)G[0]; o.g[1] = (double)G[1]; o.g[2] = (double)G[2];
   return o;
 }
@@ -784,34 +816,30 @@ __device__ __forceinline__ void k_cyc_sweep_nodes_x_body(Dims dm, const Scalars*
     const double* __restrict__ nm_in, const double* __restrict__ udin, double* __restrict__ udout,
     const double* __restrict__ dpf, double* __restrict__ Gd, const double* __restrict__ mass,
     double* __restrict__ vout, double* __restrict__ nm_out, double* __restrict__ vnorm,
-    int bx_, int by_, int bz_, double* __restrict__ ecn = nullptr) {
+    int bx_, double* __restrict__ ecn = nullptr) {
   const int lane = threadIdx.x & 31;
-  const int j = by_ * kLineWarps + (threadIdx.x >> 5), k = bz_;
-  if (j > dm.ny) return;                               // whole warp leaves together
+  if (row_first(bx_) >= (int)dm.N) return;             // whole warp leaves together
   R G[3];
   double out[LAST ? kNodeOutLast : kNodeOut];
   if constexpr (sizeof(R) == 8) {
     unsigned oor = 0u;
-    nodes_x_line<FIRST, LAST, K, R, GL, true>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, by_,
-                                              bz_, G, out, &oor);
+    nodes_x_line<FIRST, LAST, K, R, GL, true>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, G, out, &oor);
     if (__any_sync(0xffffffffu, oor != 0u)) {
       const NodeLineOut o = nodes_x_line_exact<FIRST, LAST, K, R, GL>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin,
-                                                                      dpf, Gd, mass, bx_, by_, bz_);
+                                                                      dpf, Gd, mass, bx_);
 #pragma unroll
       for (int c = 0; c < (LAST ? kNodeOutLast : kNodeOut); ++c) out[c] = o.v[c];
       G[0] = o.g[0]; G[1] = o.g[1]; G[2] = o.g[2];
     }
   } else {
-    nodes_x_line<FIRST, LAST, K, R, GL, false>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, by_,
-                                               bz_, G, out, nullptr);
+    nodes_x_line<FIRST, LAST, K, R, GL, false>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, dpf, Gd, mass, bx_, G, out, nullptr);
   }
-  const int nx = dm.nx, ny = dm.ny, N = (int)dm.N;
-  const int m = bx_ * kLineUpd - 2 + lane;
-  const bool upd = m >= 0 && m <= nx && lane >= 2 && lane < 2 + kLineUpd;
-  const bool inner = m >= 1 && m <= nx - 1;
+  const int nx = dm.nx, N = (int)dm.N;
+  const RowPos rp = row_pos(bx_, nx + 1, dm.ny + 1, N);
+  const bool upd = rp.valid && lane >= 2 && lane < 2 + kLineUpd;
+  const bool inner = rp.s >= 1 && rp.s <= nx - 1;
   const bool grad_on = ph.ordre_projection > 1;
-  const int idx[3] = {m, j, k};
-  const int n = m + (nx + 1) * (j + (ny + 1) * k);
+  const int idx[3] = {rp.s, rp.j, rp.k}, n = rp.id;
   if (!upd) return;
   if (inner && grad_on && node_on_plane(dm, 0, idx)) { Gd[n] = (double)G[0]; Gd[N + n] = (double)G[1]; Gd[2 * N + n] = (double)G[2]; }
   if (!LAST) {
@@ -829,7 +857,7 @@ __global__ void __launch_bounds__(32 * kLineWarps, kLineMinBlocks) k_cyc_sweep_n
     const double* __restrict__ nm_in, const double* __restrict__ udin, double* __restrict__ udout,
     const double* __restrict__ dpf, double* __restrict__ Gd, const double* __restrict__ mass,
     double* __restrict__ vout, double* __restrict__ nm_out, double* __restrict__ vnorm, double* __restrict__ ecn) {
-  k_cyc_sweep_nodes_x_body<FIRST, LAST, K, R, GL>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, udout, dpf, Gd, mass, vout, nm_out, vnorm, blockIdx.x, blockIdx.y, blockIdx.z, ecn);
+  k_cyc_sweep_nodes_x_body<FIRST, LAST, K, R, GL>(dm, S, ph, prev_inner, x0, xl, vh, nm_in, udin, udout, dpf, Gd, mass, vout, nm_out, vnorm, blockIdx.x, ecn);
 }
 
 // Node sweep along y (D = 1) or z (D = 2), staged through shared memory.

@@ -546,12 +546,11 @@ static void sweep_nodes_launch_w(const CycleArgs& a, int prev, const double* udi
 template <int D, bool FIRST, bool LAST, int K, typename R>
 static void sweep_nodes_launch(const CycleArgs& a, int prev, const double* udin, double* udout, cudaStream_t s) {
   const Dims& dm = a.dm;
-  const int nseg = (dm.ncd(D) + 1 + kLineUpd - 1) / kLineUpd;
   const int T = 32 * kLineWarps;
   // the generalised limiters (FP64) have their own kernels
   const bool gl = sizeof(R) == 8 && a.ph.ordre_projection > 1 && a.ph.limiteur_id >= 3;
   if constexpr (D == 0) {
-    const dim3 g(nseg, (dm.ny + 1 + kLineWarps - 1) / kLineWarps, dm.nz + 1);
+    const int g = row_chunks(dm.N);
     if (gl)
       k_cyc_sweep_nodes_x<FIRST, LAST, K, R, true><<<g, T, 0, s>>>(dm, a.S, a.ph, prev, a.x0, a.xl, a.vh, a.nm, udin,
                                                                 udout, a.dpf, a.Gd, a.st.mass, a.v, a.nm, a.vnorm, a.ecn);

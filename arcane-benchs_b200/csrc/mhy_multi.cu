@@ -1117,7 +1117,7 @@ __global__ void __launch_bounds__(32 * kLineWarps, kLineMinBlocks) k_bat_env_nod
     // schema-csts: the forward velocity on the Lagrangian coordinates (xl is null otherwise)
     k_cyc_sweep_nodes_x_body<FIRST, LAST, K, R, GL>(a.dm, a.S, a.ph, prev, a.x0, a.xl, a.ph.csts ? a.vf : a.vh, a.nm,
                                                  a.ud[(it + 1) & 1], a.ud[it & 1], a.dpf, a.Gd, a.st.mass, a.v, a.nm,
-                                                 a.vnorm, t.y, t.z, t.w, a.ecn);
+                                                 a.vnorm, t.y, a.ecn);
   }
 }
 

@@ -2,11 +2,14 @@
 its remainders change.  The cycle graph below 131072 cells runs node and cell
 sweeps side by side; a batch, which never does, must give the same bits.  The
 allocation-free dt runs as one cluster up to 8192 segments of 4 layers, else over
-segments of 4 or 8; the value is compared with its definition."""
+segments of 4 or 8; the value is compared with its definition.  The x sweeps
+take rows as one sequence of 28 updated items a warp: rows shorter and longer
+than that, against the oracle."""
 import numpy as np
 import pytest
 
 import mhy_b200
+import mhy_oracle
 from mhy_b200 import Batch, Context, gen
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +66,20 @@ def test_allocation_free_dt_is_the_minimum_of_its_definition(n):
     dev[0][-1, -1, -1] = -1.0                         # the last cell inverted
     got = call()
     assert np.isnan(got[0]) and got[1] == 0.0
+
+
+@pytest.mark.parametrize("n", [(2, 5, 3), (3, 2, 2), (27, 3, 4), (28, 9, 2), (29, 4, 5), (56, 3, 3), (61, 7, 2)])
+@pytest.mark.parametrize("limiter", [0, 2, 5])
+def test_rows_of_any_length_bitwise(n, limiter):
+    if limiter >= 3 and min(n) < 3:                   # the generalised limiters need 3 cells a direction
+        n = tuple(max(x, 3) for x in n)
+    case = gen.sod(*n, lx=n[0] * 0.01, ly=n[1] * 0.01, lz=n[2] * 0.01, jitter=0.02, seed=4,
+                   options=gen.Options(projection_limiteur_id=limiter))
+    o, g = mhy_oracle.Oracle(case, pow_mode="project"), Context(case, device=0)
+    for _ in range(9):                                # three rotations of the sweep order
+        o.step(1)
+        g.step(1)
+    g.synchronize()
+    for f in FIELDS:
+        assert np.array_equal(o.field(f), g.field(f)), f
+    assert o.scalars()["dt"] == g.dt()[0]
