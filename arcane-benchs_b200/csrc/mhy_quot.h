@@ -4,7 +4,10 @@
 // From P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34(1), 1990:
 //   - if y1 is within one ulp of 1/y, then e = 1 - y y1 is exact with one fma
-//     and RN(y1 + y1 e) = RN(1/y), unless the significand of y is all ones;
+//     and RN(y1 + y1 e) = RN(1/y), unless the significand of y is all ones:
+//     1/y is then just above the middle between a power of two and the next
+//     number, so RN(1/y) is that next number, and setting the last bit of
+//     either neighbour gives it;
 //   - with r = RN(1/y), q0 = RN(x r) and e = x - y q0 (exact with one fma),
 //     RN(q0 + e r) = RN(x/y),
 // as long as nothing underflows or overflows.  y1 comes from a seed y0 of
@@ -14,9 +17,9 @@
 // The range: 2^-960 <= |x|, |q0| < 2^960 for a nonzero x and 2^-959 <= |y| <
 // 2^960, all tested on the exponents: the residual of the quotient is then a
 // multiple of 2^-1065 and nothing overflows.  Where an operand leaves the range
-// (zero y, subnormals, infinities, NaN) or the significand of y is all ones,
-// bad gets a nonzero value and the caller computes x / y again.  8e9 random
-// and adversarial pairs that raised nothing agreed with x / y and 1 / y.
+// (zero y, subnormals, infinities, NaN), bad gets a nonzero value and the
+// caller computes x / y again.  8e9 random and adversarial pairs that raised
+// nothing agreed with x / y and 1 / y.
 //
 // Why: the compiler's division takes a branch to a slow path at every quotient,
 // so the independent quotients of a sweep (FP64 results take tens of cycles)

@@ -329,7 +329,9 @@ typedef struct mhy_tuning {
                                               1..100 (100) */
   int32_t lines_per_block[MHY_TUNE_SLOTS]; /* slots 3, 4, 6, 7 (y/z sweeps) of one-environment meshes: 8 (default),
                                               16 or 32 lines of 32 positions per block, i.e. rows of 64, 128 or
-                                              256 contiguous bytes in the staged loads; other slots 8 */
+                                              256 contiguous bytes in the staged loads; other slots 8.  A sweep
+                                              that marches (large meshes: one thread walks a piece of a line)
+                                              takes pieces of up to 2 x this many */
   double ms_default[MHY_TUNE_SLOTS];       /* autotune: measured ms per cycle of each slot with the defaults ... */
   double ms_tuned[MHY_TUNE_SLOTS];         /* ... and with the chosen settings */
   int32_t from_cache;                      /* 1: taken from the in-process cache (keyed on the mesh sizes, the
