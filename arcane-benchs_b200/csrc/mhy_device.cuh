@@ -68,6 +68,13 @@ __device__ __forceinline__ R rc(R y, unsigned* oor) {
   if constexpr (sizeof(R) == 8 && SP) return rcp_fast(y, *oor);
   else return R(1) / y;
 }
+// The same with the plain reciprocal, for kernels at the register limit, where
+// rcp_fast spills: the speculative form adds the check of y that dv relies on.
+template <typename R, bool SP>
+__device__ __forceinline__ R rc_plain(R y, unsigned* oor) {
+  if constexpr (sizeof(R) == 8 && SP) return rcp_checked(y, *oor);
+  else return R(1) / y;
+}
 template <typename R, bool SP>
 __device__ __forceinline__ R dv(R x, R y, R r, unsigned* oor) {
   if constexpr (sizeof(R) == 4) return x * r;

@@ -65,7 +65,7 @@ __device__ __forceinline__ void face_values_env(const Phys& ph, int lim, bool in
   const double dx = inner ? dot(d3(in.xc[0], in.xc[1], in.xc[2]) - d3(xpx, xpy, xpz), d3(in.n[0], in.n[1], in.n[2]))
                           : 0.;
   unsigned fo = 0u;
-  const R dxR = (R)dx, rdx = inner ? R(1) / dxR : R(0);
+  const R dxR = (R)dx, rdx = inner ? rc_plain<R, SP>(dxR, &fo) : R(0);
   R G[NV], Pp[NV];
   R h0 = R(0), hm = R(0), hp = R(0);
   if constexpr (GL) {
@@ -203,7 +203,7 @@ __device__ __forceinline__ void cell_line_env(const Phys& ph, double dt, bool va
 #pragma unroll
           for (int k = 0; k < K; ++k) den += in.U[k];
         }
-        const R dR = (R)den, r = R(1) / dR;
+        const R dR = (R)den, r = rc_plain<R, SP>(dR, oor);
 #pragma unroll
         for (int v = 0; v < NV; ++v) P[v] = dv<R, SP>((R)in.U[v], dR, r, oor);
       }

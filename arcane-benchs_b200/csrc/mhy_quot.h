@@ -84,7 +84,18 @@ MHY_Q_HD double rcp_from_seed(double y, double y0, unsigned& bad) {
   return q_make(q_hi(r), q_lo(r) | ones);
 }
 
-// RN(x/y) with r = RN(1/y); a zero x gives the zero of the right sign (q0's).
+// The plain 1 / y with the check of y that quo_from_rcp leaves to whoever forms r.
+MHY_Q_HD double rcp_checked(double y, unsigned& bad) {
+  const uint32_t h = q_hi(y);
+  if (MHY_Q_OUT(h, 64, 1983)) bad = 1u;
+  return 1.0 / y;
+}
+
+// RN(x/y) with r = RN(1/y) of a y inside the range: whoever formed r has raised
+// bad for any other y (rcp_from_seed and rcp_checked do).  Only x and q0 are
+// tested here, and that does not see every y outside the range: a zero x over a
+// y whose 1/y is 0 or infinite gives NaN.  A zero x gives the zero of the right
+// sign (q0's).
 MHY_Q_HD double quo_from_rcp(double x, double y, double r, unsigned& bad) {
   const double q0 = x * r;
   const double q = q_fma(q_fma(-q0, y, x), r, q0);
