@@ -901,7 +901,10 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
       b->plan.o3nwork[d] = (int)w.size();
     }
   }
-  for (int i = 0; i < n; ++i) b->plan.cons_ec |= opts[i].conservation_energie_totale;
+  for (int i = 0; i < n; ++i) {
+    b->plan.cons_ec |= opts[i].conservation_energie_totale;
+    b->plan.newton |= opts[i].with_newton;
+  }
   for (int k = 0; k < BK_TUNE_SLOTS; ++k) {
     b->plan.occ_pct[k] = 100;
     b->tuning.occupancy_pct[k] = 100;

@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(128, 3) k_cyc_lagrange_cells_csts(Dims dm,
     double* __restrict__ cqs, double* __restrict__ L, double* __restrict__ U,
     double* __restrict__ xcs, FaceData fd, EnvState env, double* __restrict__ Vlag, int linear,
     const double* __restrict__ vnb, double* __restrict__ pf) {
-  k_cyc_lagrange_cells_body<K, double, true, HC>(dm, S, ph, x0, vh, n0, rho, e, q, p, cs, mass, cqs, nullptr, L, U, xcs, fd,
+  k_cyc_lagrange_cells_body<K, double, true, HC, false>(dm, S, ph, x0, vh, n0, rho, e, q, p, cs, mass, cqs, nullptr, L, U, xcs, fd,
                                              env, Vlag, blockIdx.x, linear ? -1 : (int)blockIdx.y, blockIdx.z, vnb, pf);
 }
 
@@ -1098,8 +1098,10 @@ void launch_batch_cycle(const BatchPlan& P, int sens, cudaStream_t s, KernelMark
   launch_bat_lagrange_nodes(P, s, m);
   const bool hc = P.gl || P.pb || P.o3;   // the G limiters, pente-borne, order 3: the cell widths too
   if (P.csts || P.precision) {
-    auto kern = P.precision ? k_bat_lagrange_cells<1, float, false, false>
-                            : (hc ? k_bat_lagrange_cells<1, double, true, true> : k_bat_lagrange_cells<1, double, false, true>);
+    auto kern = P.precision ? (P.newton ? k_bat_lagrange_cells<1, float, false, false, true>
+                                        : k_bat_lagrange_cells<1, float, false, false, false>)
+                            : (hc ? k_bat_lagrange_cells<1, double, true, true, false>
+                                  : k_bat_lagrange_cells<1, double, false, true, false>);
     launch_persistent(kern, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
   } else if (hc) launch_bat_columns<1, true>(P, s, m);
   else launch_bat_columns<1, false>(P, s, m);

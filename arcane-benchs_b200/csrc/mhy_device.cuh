@@ -293,13 +293,27 @@ __device__ __forceinline__ double newton_eint(bool pc, int kind, double g, doubl
   return e;
 }
 
+// The same as a call, for the branch-free cell kernels: in line at each of the
+// K + 1 updates of a cell of K environments it would double their code.
+static __device__ __noinline__ double newton_eint_call(bool pc, int kind, double g, double pinf, double epsilon,
+                                                       double qn, double q, double ir, double irn, double r, double pn,
+                                                       double en) {
+  return newton_eint(pc, kind, g, pinf, epsilon, qn, q, ir, irn, r, pn, en);
+}
+
 // The Lagrange energy update of one environment cell: the closed form of
-// updateEnergyAndPressureforGP, or the Newton iterations when with-newton is set.
-template <bool SP = false>
+// updateEnergyAndPressureforGP, or the Newton iterations when with-newton is
+// set.  SP: the closed form's quotient is branch-free (Newton iterates with plain
+// ones), and Newton is there only in kernels built for it (NEWTON).
+template <bool SP, bool NEWTON>
 __device__ __forceinline__ double energy_update(bool newton, bool pc, int kind, double g, double pinf, double epsilon,
                                                 double qn, double q, double ir, double irn, double r, double p,
-                                                double en, unsigned* oor = nullptr) {
-  if (newton) return newton_eint(pc, kind, g, pinf, epsilon, qn, q, ir, irn, r, p, en);
+                                                double en, unsigned* oor) {
+  if constexpr (!SP) {
+    if (newton) return newton_eint(pc, kind, g, pinf, epsilon, qn, q, ir, irn, r, p, en);
+  } else if constexpr (NEWTON) {
+    if (newton) return newton_eint_call(pc, kind, g, pinf, epsilon, qn, q, ir, irn, r, p, en);
+  }
   return compute_eint<SP>(pc, g, qn, q, ir, irn, r, p, en, oor);
 }
 

@@ -199,6 +199,7 @@ struct BatchPlan {
   int pb;                       // every instance takes projection-pente-borne (FP64): the PB cell sweeps
   int o3;                       // every instance takes order 3 (FP64): face values, then the O3 cell sweeps
   int csts;                     // every instance takes schema-csts (FP64)
+  int newton;                   // an instance takes the Newton energy update
   const int4* cwork;            // the Lagrange cell kernel's columns (instance, chunk, segment); not schema-csts
   int ncwork;
   int col_strip;                // the longest strip of nodes its instances need

@@ -219,7 +219,7 @@ __device__ __forceinline__ double csts_eint(const Phys& ph, double g, int eos, d
 // kernel of Sedov 128^3 377 -> 323 us in FP64, 230 -> 219 us in the mixed form.
 struct ThermoIn { double V, inv_dt, rn, m, cs, p, q, e; };
 struct ThermoOut { double L, nd, qn, en, pf; };
-template <bool CSTS, bool F32, bool SP>
+template <bool CSTS, bool F32, bool SP, bool NEWTON>
 __device__ __forceinline__ ThermoOut thermo_one(const Phys& ph, const ThermoIn& in, double Lface, double cn1, double cn,
                                                 double cdn, double con, unsigned* oor) {
   ThermoOut o;
@@ -245,17 +245,15 @@ __device__ __forceinline__ ThermoOut thermo_one(const Phys& ph, const ThermoIn& 
   o.qn = qn;
   if constexpr (CSTS)
     o.en = csts_eint(ph, g, ph.eos, ph.pinf, cn1, cn, cdn, con, in.e, nd, in.m, in.p, in.q, qn, o.pf);
-  else if constexpr (SP)   // Newton takes the exact form
-    o.en = compute_eint<true>(ph.pseudo_centree != 0, g, in.q, qn, ind, irn, nd, in.p, in.e, oor);
   else
-    o.en = energy_update(ph.with_newton != 0, ph.pseudo_centree != 0, ph.eos, g, ph.pinf, ph.threshold, in.q, qn, ind,
-                         irn, nd, in.p, in.e);
+    o.en = energy_update<SP, NEWTON>(ph.with_newton != 0, ph.pseudo_centree != 0, ph.eos, g, ph.pinf, ph.threshold,
+                                     in.q, qn, ind, irn, nd, in.p, in.e, oor);
   return o;
 }
 template <bool CSTS, bool F32>
 __device__ __noinline__ ThermoOut thermo_one_exact(Phys ph, ThermoIn in, double Lface, double cn1, double cn, double cdn,
                                                    double con) {
-  return thermo_one<CSTS, F32, false>(ph, in, Lface, cn1, cn, cdn, con, nullptr);
+  return thermo_one<CSTS, F32, false, true>(ph, in, Lface, cn1, cn, cdn, con, nullptr);
 }
 
 // Lagrange thermodynamics of a mesh with K > 1 environments, then the remap
@@ -279,7 +277,7 @@ __device__ __noinline__ ThermoOut thermo_one_exact(Phys ph, ThermoIn in, double 
 // rn: the density before the step.  SP: the quotients of mhy_quot.h (see
 // thermo_one); where *oor is raised the cell is done again by
 // lagrange_thermo_env_exact, which writes all of it anew.
-template <int K, bool CSTS, bool SP>
+template <int K, bool CSTS, bool SP, bool NEWTON>
 __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const EnvState& env, int c, int C,
                                                     const ThermoIn& in, double Lc, double* __restrict__ rho,
                                                     double* __restrict__ U,
@@ -309,9 +307,8 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const EnvSta
                      in.p, in.q, qn, pforward);
       pf[c] = pforward + qn;
     } else {
-      en = SP ? compute_eint<SP>(pc, g, in.q, qn, ind, irn, nd, in.p, in.e, oor)
-              : energy_update(ph.with_newton != 0, pc, env.eos[ke], g, env.pinf[ke], ph.threshold, in.q, qn, ind, irn,
-                              nd, in.p, in.e);
+      en = energy_update<SP, NEWTON>(ph.with_newton != 0, pc, env.eos[ke], g, env.pinf[ke], ph.threshold, in.q, qn, ind,
+                                     irn, nd, in.p, in.e, oor);
     }
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -342,9 +339,8 @@ __device__ __forceinline__ void lagrange_thermo_env(const Phys& ph, const EnvSta
                        env.p[o], env.q[o], qk, pk_unused);
         qg += qk * env.f[o];
       } else {
-        ek = SP ? compute_eint<SP>(pc, g, env.q[o], qk, irk, irnk, rk, env.p[o], env.e[o], oor)
-                : energy_update(ph.with_newton != 0, pc, env.eos[k], g, env.pinf[k], ph.threshold, env.q[o], qk, irk,
-                                irnk, rk, env.p[o], env.e[o]);
+        ek = energy_update<SP, NEWTON>(ph.with_newton != 0, pc, env.eos[k], g, env.pinf[k], ph.threshold, env.q[o], qk,
+                                       irk, irnk, rk, env.p[o], env.e[o], oor);
       }
       u[k] = vk;
       u[K + k] = vk * rk;
@@ -365,20 +361,25 @@ template <int K, bool CSTS>
 __device__ __noinline__ void lagrange_thermo_env_exact(Phys ph, EnvState env, int c, int C, ThermoIn in, double Lc,
     double* rho, double* U, double* Vlag, double* pbphi, double cn1, double cn, double cdn, double con, double* pf) {
   const double cssum[4] = {cn1, cn, cdn, con};
-  lagrange_thermo_env<K, CSTS, false>(ph, env, c, C, in, Lc, rho, U, Vlag, pbphi, cssum, pf, nullptr);
+  lagrange_thermo_env<K, CSTS, false, true>(ph, env, c, C, in, Lc, rho, U, Vlag, pbphi, cssum, pf, nullptr);
 }
 
 // The characteristic length and the thermodynamics of a cell, then its remap
 // variables, whichever number of environments.  Lface: the length of
-// faces-opposees (used when lc_mode is 1).
-template <int K, bool CSTS, bool F32>
+// faces-opposees (used when lc_mode is 1).  NEWTON: the kernels of contexts with
+// with-newton, and of batches with an instance that has it.  Measured on B200:
+// one kernel for both spills (two gases 256x128x128 without Newton 2.74 -> 2.81 ms
+// a cycle); Newton by way of the exact form costs a copy of its arguments and plain
+// quotients in every cell (a cycle with Newton 3.14 ms there and 460 us with three
+// gases on 90x60x60, 2.89 ms and 405 us in these kernels).
+template <int K, bool CSTS, bool F32, bool NEWTON>
 __device__ __forceinline__ void cell_thermo(const Phys& ph, const EnvState& env, const FaceData& fd, int c, int C,
                                             const ThermoIn& in, double Lface, double* __restrict__ rho,
                                             double* __restrict__ L, double* __restrict__ U, double* __restrict__ Vlag,
                                             double cn1, double cn, double cdn, double con, double* __restrict__ pf) {
-  unsigned oor = ph.with_newton && !CSTS ? 1u : 0u;   // Newton iterates with plain quotients
+  unsigned oor = 0u;
   if constexpr (K == 1) {
-    ThermoOut t = thermo_one<CSTS, F32, true>(ph, in, Lface, cn1, cn, cdn, con, &oor);
+    ThermoOut t = thermo_one<CSTS, F32, true, NEWTON>(ph, in, Lface, cn1, cn, cdn, con, &oor);
     if (oor) t = thermo_one_exact<CSTS, F32>(ph, in, Lface, cn1, cn, cdn, con);
     L[c] = t.L;
     if constexpr (CSTS) pf[c] = t.pf + t.qn;                      // the forward force's p + q (q: this cycle's)
@@ -399,8 +400,7 @@ __device__ __forceinline__ void cell_thermo(const Phys& ph, const EnvState& env,
     }
     L[c] = Lc;
     const double cssum[4] = {cn1, cn, cdn, con};
-    if (!oor)
-      lagrange_thermo_env<K, CSTS, true>(ph, env, c, C, in, Lc, rho, U, Vlag, fd.pbphi, cssum, pf, &oor);
+    lagrange_thermo_env<K, CSTS, true, NEWTON>(ph, env, c, C, in, Lc, rho, U, Vlag, fd.pbphi, cssum, pf, &oor);
     if (oor)
       lagrange_thermo_env_exact<K, CSTS>(ph, env, c, C, in, Lc, rho, U, Vlag, fd.pbphi, cn1, cn, cdn, con, pf);
   }
@@ -416,7 +416,7 @@ __device__ __forceinline__ double face_length(const D3 x[8]) {
 
 // CSTS (schema-csts, FP64 only): vnb = the backward node velocity of this
 // cycle, pf = the pressure plus pseudo-viscosity of the forward step.
-template <int K, typename R, bool CSTS = false, bool HC = false>
+template <int K, typename R, bool CSTS, bool HC, bool NEWTON>
 __device__ __forceinline__ void k_cyc_lagrange_cells_body(Dims dm, const Scalars* __restrict__ S, Phys ph,
     const double* __restrict__ x0, const double* __restrict__ vh, const double* __restrict__ n0,
     double* __restrict__ rho, const double* __restrict__ e, const double* __restrict__ q,
@@ -501,7 +501,7 @@ __device__ __forceinline__ void k_cyc_lagrange_cells_body(Dims dm, const Scalars
     }
   }
   const ThermoIn in{V, S->inv_dt, rho[c], mass[c], cs[c], p[c], q[c], e[c]};
-  cell_thermo<K, CSTS, F32>(ph, env, fd, (int)c, (int)C, in, Lc, rho, L, U, Vlag, cs_cn1, cs_cn, cs_cdn, cs_con, pf);
+  cell_thermo<K, CSTS, F32, NEWTON>(ph, env, fd, (int)c, (int)C, in, Lc, rho, L, U, Vlag, cs_cn1, cs_cn, cs_cdn, cs_con, pf);
   auto normal = [&](long long f) { return d3(n0[f], n0[dm.F + f], n0[2 * dm.F + f]); };
   auto nlo = [&](int d) { return normal(dm.fid(d, i, j, k)); };
   auto nhi = [&](int d) { return normal(dm.fid(d, i + (d == 0), j + (d == 1), k + (d == 2))); };
@@ -513,7 +513,7 @@ __device__ __forceinline__ void k_cyc_lagrange_cells_body(Dims dm, const Scalars
   else face_data<double, HC>(dm, i, j, k, x, xc, fd, nlo, nhi, vn);
 }
 
-template <int K, typename R, bool HC = false>
+template <int K, typename R, bool HC, bool NEWTON>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_cyc_lagrange_cells(Dims dm,
     const Scalars* __restrict__ S, Phys ph,
     const double* __restrict__ x0, const double* __restrict__ vh, const double* __restrict__ n0,
@@ -521,8 +521,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_cyc_lagrange_ce
     const double* __restrict__ p, const double* __restrict__ cs, const double* __restrict__ mass,
     double* __restrict__ cqs, float* __restrict__ cqs32, double* __restrict__ L, double* __restrict__ U,
     double* __restrict__ xcs, FaceData fd, EnvState env, double* __restrict__ Vlag, int linear) {
-  k_cyc_lagrange_cells_body<K, R, false, HC>(dm, S, ph, x0, vh, n0, rho, e, q, p, cs, mass, cqs, cqs32, L, U, xcs, fd,
-                                             env, Vlag, blockIdx.x, linear ? -1 : (int)blockIdx.y, blockIdx.z);
+  k_cyc_lagrange_cells_body<K, R, false, HC, NEWTON>(dm, S, ph, x0, vh, n0, rho, e, q, p, cs, mass, cqs, cqs32, L, U,
+                                                     xcs, fd, env, Vlag, blockIdx.x, linear ? -1 : (int)blockIdx.y, blockIdx.z);
 }
 
 // ------------------------------------------------------------------------
@@ -560,7 +560,7 @@ __device__ __forceinline__ void cp_async8(double* s, const double* g) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
 template <int Left> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(Left) : "memory"); }
 
-template <int K, bool HC, int strip>
+template <int K, bool HC, int strip, bool NEWTON>
 __device__ __forceinline__ void lagrange_columns(const CycleArgs& A, int bx, int seg) {
   extern __shared__ double col_mem[];
   const Dims& dm = A.dm;
@@ -679,21 +679,22 @@ __device__ __forceinline__ void lagrange_columns(const CycleArgs& A, int bx, int
       double Lc = 0.;
       A.xc[c] = xc.x; A.xc[C + c] = xc.y; A.xc[2 * C + c] = xc.z;
       if (A.ph.lc_mode != 0) Lc = face_length(x);
-      cell_thermo<K, false, false>(A.ph, A.env, A.fd, c, C, in, Lc, A.st.rho, A.L, A.U[0], A.Vlag, 0., 0., 0., 0., nullptr);
+      cell_thermo<K, false, false, NEWTON>(A.ph, A.env, A.fd, c, C, in, Lc, A.st.rho, A.L, A.U[0], A.Vlag, 0., 0., 0.,
+                                           0., nullptr);
       face_data<double, HC>(dm, i, j, k, x, xc, A.fd, nlo, nhi, vn);
     }
   }
 }
 
-template <int K, bool HC, int STRIP>
+template <int K, bool HC, int STRIP, bool NEWTON>
 __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_cyc_lagrange_columns(const __grid_constant__ CycleArgs a) {
-  lagrange_columns<K, HC, STRIP>(a, blockIdx.x, blockIdx.y);
+  lagrange_columns<K, HC, STRIP, NEWTON>(a, blockIdx.x, blockIdx.y);
 }
 
 // The same over a batch's column table (instance, chunk, segment).  The
 // instance's arguments are read from shared memory where they are used:
 // fifty pointers in registers would spill.
-template <int K, bool HC, int STRIP>
+template <int K, bool HC, int STRIP, bool NEWTON>
 __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat_lagrange_columns(const CycleArgs* __restrict__ D,
                                                                          const int4* __restrict__ W, int nw) {
   __shared__ CycleArgs a;
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat
     for (int x = threadIdx.x; x < (int)(sizeof(CycleArgs) / sizeof(double)); x += kColThreads)
       reinterpret_cast<double*>(&a)[x] = reinterpret_cast<const double*>(D + t.x)[x];
     __syncthreads();
-    lagrange_columns<K, HC, STRIP>(a, t.y, t.z);
+    lagrange_columns<K, HC, STRIP, NEWTON>(a, t.y, t.z);
   }
 }
 
@@ -713,51 +714,64 @@ __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat
 // 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1).
 constexpr long long kColMinCells = 65536;
 
-template <int K, bool HC>
+template <int K, bool HC, bool NEWTON>
 static void launch_columns(const CycleArgs& a, cudaStream_t s) {
   const Dims& dm = a.dm;
   const int strip = col_strip(dm.nx);
   const size_t smem = col_smem(strip);
-  auto kern = strip == kColStrip ? k_cyc_lagrange_columns<K, HC, kColStrip> : k_cyc_lagrange_columns<K, HC, kColStripWide>;
+  auto kern = strip == kColStrip ? k_cyc_lagrange_columns<K, HC, kColStrip, NEWTON>
+                                 : k_cyc_lagrange_columns<K, HC, kColStripWide, NEWTON>;
   smem_opt_in((const void*)kern, smem);
   kern<<<dim3(col_blocks(dm.nx, dm.ny), col_segments(dm.nx, dm.ny, dm.nz)), kColThreads, smem, s>>>(a);
 }
 
 // The cell kernel of a context, all but schema-csts.
-template <int K>
+template <int K, bool NEWTON>
 static void launch_cells(const CycleArgs& a, cudaStream_t s) {
   const bool hc = a.fd.h != nullptr;               // cell widths: order 3 or the generalised limiters
   if (!a.ph.precision && a.dm.C >= kColMinCells) {
-    if (hc) launch_columns<K, true>(a, s);
-    else launch_columns<K, false>(a, s);
+    if (hc) launch_columns<K, true, NEWTON>(a, s);
+    else launch_columns<K, false, NEWTON>(a, s);
     return;
   }
   int linear;
   const dim3 nbc = cell_grid(a.dm, linear);
-  auto kern = a.ph.precision ? k_cyc_lagrange_cells<K, float> : (hc ? k_cyc_lagrange_cells<K, double, true> : k_cyc_lagrange_cells<K, double>);
+  auto kern = a.ph.precision ? k_cyc_lagrange_cells<K, float, false, NEWTON>
+                             : (hc ? k_cyc_lagrange_cells<K, double, true, NEWTON> : k_cyc_lagrange_cells<K, double, false, NEWTON>);
   kern<<<nbc, 128, 0, s>>>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p, a.st.cs, a.st.mass,
                            a.cqs, a.cqs32, a.L, a.U[0], a.xc, a.fd, a.env, a.Vlag, linear);
 }
+template <int K>
+static void launch_cells(const CycleArgs& a, cudaStream_t s) {
+  if (a.ph.with_newton) launch_cells<K, true>(a, s);
+  else launch_cells<K, false>(a, s);
+}
 
-template <int K, bool HC>
+template <int K, bool HC, bool NEWTON>
 static void launch_bat_columns(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
   const size_t smem = col_smem(P.col_strip);
-  auto kern = P.col_strip == kColStrip ? k_bat_lagrange_columns<K, HC, kColStrip> : k_bat_lagrange_columns<K, HC, kColStripWide>;
+  auto kern = P.col_strip == kColStrip ? k_bat_lagrange_columns<K, HC, kColStrip, NEWTON>
+                                       : k_bat_lagrange_columns<K, HC, kColStripWide, NEWTON>;
   smem_opt_in((const void*)kern, smem);
   if (P.ncwork > 0)
     kern<<<persistent_grid((const void*)kern, kColThreads, smem, P.ncwork, P.occ_pct[BK_LCELLS]), kColThreads, smem, s>>>(
         P.descs, P.cwork, P.ncwork);
   mark(m, BK_LCELLS, s);
 }
+template <int K, bool HC>
+static void launch_bat_columns(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  if (P.newton) launch_bat_columns<K, HC, true>(P, s, m);
+  else launch_bat_columns<K, HC, false>(P, s, m);
+}
 
 // A batch's mixed form and schema-csts: the cell tiles of BK_LCELLS.
-template <int K, typename R, bool HC, bool CSTS>
+template <int K, typename R, bool HC, bool CSTS, bool NEWTON>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_lagrange_cells(const CycleArgs* __restrict__ D,
                                                                                    const int4* __restrict__ W, int nw) {
   for (int w = blockIdx.x; w < nw; w += gridDim.x) {
     const int4 t = W[w];
     const CycleArgs& a = D[t.x];
-    k_cyc_lagrange_cells_body<K, R, CSTS, HC>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p,
+    k_cyc_lagrange_cells_body<K, R, CSTS, HC, NEWTON>(a.dm, a.S, a.ph, a.x0, a.vh, a.n0, a.st.rho, a.st.e, a.st.q, a.st.p,
                                               a.st.cs, a.st.mass, a.cqs, CSTS ? nullptr : a.cqs32, a.L, a.U[0], a.xc,
                                               a.fd, a.env, a.Vlag, t.y, t.z, t.w, a.vnb, a.pf);
   }
