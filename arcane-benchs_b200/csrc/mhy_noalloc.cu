@@ -124,8 +124,9 @@ __device__ __forceinline__ unsigned long long block_min(unsigned long long best,
 // where a value is NaN or negative.  The maximum is taken over |v|^2, in the
 // cell-node order, with one root a cell: the root is monotonic, so its result
 // is the maximum of the roots.  The four nodes of a layer's top are the next
-// layer's bottom.  Four layers are loaded before the first root and division,
+// layer's bottom.  Q (four) layers are loaded before the first root and division,
 // whose branches would keep the loads apart.
+template <int Q>
 __device__ __forceinline__ unsigned long long column_dt_min(const Dims& dm, const double* __restrict__ L,
                                                             const double* __restrict__ cs,
                                                             const double* __restrict__ v, int p, int k0, int k1,
@@ -144,10 +145,10 @@ __device__ __forceinline__ unsigned long long column_dt_min(const Dims& dm, cons
   };
   double b[4];
   plane(k0, b);
-  for (int k = k0; k < k1; k += 4) {
-    double vmax[4], lc[4], cc[4];
+  for (int k = k0; k < k1; k += Q) {
+    double vmax[Q], lc[Q], cc[Q];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < Q; ++q) {
       const int kq = k + q < k1 ? k + q : k1 - 1;   // past the end the last cell again
       double t[4];
       plane(kq + 1, t);
@@ -164,7 +165,7 @@ __device__ __forceinline__ unsigned long long column_dt_min(const Dims& dm, cons
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < Q; ++q) {
       const double dx_sound = lc[q] / (cc[q] + sqrt(vmax[q]));
       const unsigned long long bits = (unsigned long long)__double_as_longlong(dx_sound);
       if (dx_sound >= 0.) best = bits < best ? bits : best;
@@ -194,6 +195,7 @@ __device__ __forceinline__ void write_dt(unsigned long long best, bool bad, doub
 // The minimum over this block's part of the mesh (valid in thread 0), with
 // kInvalidBit set when the block met a NaN or negative value.  A thread walks
 // segments of `layers` layers of a column, a grid apart.
+template <int Q>
 __device__ __forceinline__ unsigned long long block_partial(const Dims& dm, const double* __restrict__ L,
                                                             const double* __restrict__ cs,
                                                             const double* __restrict__ v, int layers) {
@@ -208,7 +210,7 @@ __device__ __forceinline__ unsigned long long block_partial(const Dims& dm, cons
   for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < items; w += gridDim.x * blockDim.x) {
     const int seg = (int)(w / points), p = (int)(w - seg * points), k0 = seg * layers;
     const int k1 = k0 + layers < dm.nz ? k0 + layers : dm.nz;
-    const unsigned long long b = column_dt_min(dm, L, cs, v, p, k0, k1, invalid);
+    const unsigned long long b = column_dt_min<Q>(dm, L, cs, v, p, k0, k1, invalid);
     best = b < best ? b : best;
   }
   if (invalid) bad = 1;                             // benign race: every writer stores 1
@@ -217,21 +219,23 @@ __device__ __forceinline__ unsigned long long block_partial(const Dims& dm, cons
 }
 
 // First pass: one partial minimum per block.
+template <int Q>
 __global__ void __launch_bounds__(kNoAllocThreads) k_dt_partial_noalloc(Dims dm, const double* __restrict__ L,
     const double* __restrict__ cs, const double* __restrict__ v, int layers, unsigned long long* __restrict__ scratch) {
-  const unsigned long long best = block_partial(dm, L, cs, v, layers);
+  const unsigned long long best = block_partial<Q>(dm, L, cs, v, layers);
   if (threadIdx.x == 0) scratch[blockIdx.x] = best;
 }
 
 // The whole call on one cluster: its first block gathers the partial minima in
 // its shared memory.
+template <int Q>
 __global__ void __launch_bounds__(kNoAllocClusterThreads) k_dt_cluster_noalloc(Dims dm, const double* __restrict__ L,
     const double* __restrict__ cs, const double* __restrict__ v, double cfl, double dt_old, double deltat_max,
     double* __restrict__ out) {
   __shared__ unsigned long long part[kNoAllocCluster];
   auto cluster = cooperative_groups::this_cluster();
   cluster.barrier_arrive();                         // this block runs
-  unsigned long long best = block_partial(dm, L, cs, v, kNoAllocLayers);
+  unsigned long long best = block_partial<Q>(dm, L, cs, v, Q);
   cluster.barrier_wait();                           // every block runs, so its shared memory is there
   if (threadIdx.x == 0) cluster.map_shared_rank(part, 0)[blockIdx.x] = best;
   cluster.sync();
@@ -300,13 +304,27 @@ extern "C" int mhy_compute_hydro_dt_noalloc(int32_t nx, int32_t ny, int32_t nz, 
     scratch = sa.addr;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // One cluster of eight blocks where it has a thread for every segment of 4
-  // layers: a second launch costs more than eight SMs lose.  Otherwise segments
-  // of 8 layers, of 4 where those would not fill the chip (148 SMs x 8 blocks).
-  // Measured on B200, the call, against one thread a cell with its eight nodes in
-  // two launches: 100x5x5 11.9 -> 9.0 us, 32^3 11.9 -> 8.9 (two segments a thread,
-  // 40^3: 13.6 against 11.9 in two launches), 64^3 14.3 -> 11.9, 128^3 66 -> 37.
-  const long long points = (long long)nx * ny, segments = points * ((nz + kNoAllocLayers - 1) / kNoAllocLayers);
+  // A thread walks segments of 4 layers, of 8 where those still fill the chip
+  // (148 SMs x 8 blocks), and of one layer where longer ones do not pay:
+  //  * one layer of cells: there is nothing to walk, and the other three of a chunk
+  //    of four would be the same cell again (2048x1024x1 91 -> 51 us, 500x500x1 17
+  //    -> 13);
+  //  * layers of less than 4 cells: neighbouring threads would read lines that lie
+  //    a segment apart (1x1x32000 38 -> 9 us, 1x1x2000000 138 -> 78, 1x2x1000000
+  //    68 -> 57; from 4 cells on segments are ahead: 2x2x500000 50 us against 65);
+  //  * layers of less than 128 cells on meshes of 8,193 to 65,536 cells, for the same
+  //    reason while that many threads are resident at once (8x8x512 10.7 -> 8.5 us,
+  //    1x8x4090 12.6 -> 8.5; nothing between the two at 8x8x1030).
+  // One cluster of eight blocks where it has a thread for every segment: a second
+  // launch costs more than eight SMs lose.  Measured on B200, the call, against
+  // one thread a cell with its eight nodes and roots in two launches: 100x5x5 11.9
+  // -> 9.0 us, 32^3 11.9 -> 8.9, 64^3 14.3 -> 11.9, 128^3 66 -> 37, 2048x1024x1 72
+  // -> 51, 1x1x2000000 76 -> 78 (a cluster with two segments a thread, for 40^3,
+  // took 13.6 us against 11.9 in two launches and was left out).
+  const long long points = (long long)nx * ny;
+  const bool narrow = points < 128 && dm.C > 8192 && dm.C <= 65536;
+  const int q = nz == 1 || points < 4 || narrow ? 1 : kNoAllocLayers;
+  const long long segments = points * ((nz + q - 1) / q);
   if (segments <= kNoAllocCluster * kNoAllocClusterThreads) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -318,12 +336,14 @@ extern "C" int mhy_compute_hydro_dt_noalloc(int32_t nx, int32_t ny, int32_t nz, 
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_dt_cluster_noalloc, dm, L, cs, v, cfl, dt_old, deltat_max, out);
+    auto kern = q == 1 ? k_dt_cluster_noalloc<1> : k_dt_cluster_noalloc<kNoAllocLayers>;
+    cudaLaunchKernelEx(&cfg, kern, dm, L, cs, v, cfl, dt_old, deltat_max, out);
   } else {
-    const int layers = points * ((nz + 7) / 8) < 148LL * 8 * kNoAllocThreads ? kNoAllocLayers : 8;
+    const int layers = q == 1 || points * ((nz + 7) / 8) < 148LL * 8 * kNoAllocThreads ? q : 8;
     const long long want = (points * ((nz + layers - 1) / layers) + kNoAllocThreads - 1) / kNoAllocThreads;
     const int nblocks = (int)(want < kNoAllocBlocks ? want : kNoAllocBlocks);
-    k_dt_partial_noalloc<<<nblocks, kNoAllocThreads, 0, s>>>(dm, L, cs, v, layers, scratch);
+    auto first = q == 1 ? k_dt_partial_noalloc<1> : k_dt_partial_noalloc<kNoAllocLayers>;
+    first<<<nblocks, kNoAllocThreads, 0, s>>>(dm, L, cs, v, layers, scratch);
     k_dt_final_noalloc<<<1, 1024, 0, s>>>(scratch, nblocks, cfl, dt_old, deltat_max, out);
   }
   if (cudaGetLastError() != cudaSuccess) return MHY_ERR_CUDA;
