@@ -858,11 +858,15 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
     if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
     b->plan.cwork = b->d_cwork;
     b->plan.ncwork = (int)w.size();
+    long long cells = 0, threads = 0;
     for (const mhy_ctx* c : b->inst) {
       int blocks, segments, strip;
       batch_column_shape(c->dm, blocks, segments, strip);
       b->plan.col_strip = std::max(b->plan.col_strip, strip);
+      cells += c->dm.C;
+      threads += (long long)kColThreads * blocks * c->dm.nz;
     }
+    b->plan.columns = opts[0].precision == 0 && !opts[0].schema_csts && col_filled(cells, threads);
   }
   err = cudaMalloc(&b->d_descs, n * sizeof(CycleArgs));
   if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }

@@ -1097,14 +1097,11 @@ void launch_batch_cycle(const BatchPlan& P, int sens, cudaStream_t s, KernelMark
   if (P.K > 1) { launch_batch_cycle_env(P, sens, s, m); return; }
   launch_bat_lagrange_nodes(P, s, m);
   const bool hc = P.gl || P.pb || P.o3;   // the G limiters, pente-borne, order 3: the cell widths too
-  if (P.csts || P.precision) {
-    auto kern = P.precision ? (P.newton ? k_bat_lagrange_cells<1, float, false, false, true>
-                                        : k_bat_lagrange_cells<1, float, false, false, false>)
-                            : (hc ? k_bat_lagrange_cells<1, double, true, true, false>
-                                  : k_bat_lagrange_cells<1, double, false, true, false>);
-    launch_persistent(kern, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  } else if (hc) launch_bat_columns<1, true>(P, s, m);
-  else launch_bat_columns<1, false>(P, s, m);
+  if (P.precision) launch_bat_cells<1, float, false>(P, s, m);
+  else if (P.csts && hc) launch_bat_tiles<1, double, true, true, false>(P, s, m);
+  else if (P.csts) launch_bat_tiles<1, double, false, true, false>(P, s, m);
+  else if (hc) launch_bat_cells<1, double, true>(P, s, m);
+  else launch_bat_cells<1, double, false>(P, s, m);
   launch_bat_csts_forward(P, s);   // PrepareRemap.cc:456, then the face velocities
   if (P.precision) bat_sweeps<float, false>(P, sens, s, m);
   else if (P.gl) bat_sweeps<double, true>(P, sens, s, m);

@@ -200,7 +200,8 @@ struct BatchPlan {
   int o3;                       // every instance takes order 3 (FP64): face values, then the O3 cell sweeps
   int csts;                     // every instance takes schema-csts (FP64)
   int newton;                   // an instance takes the Newton energy update
-  const int4* cwork;            // the Lagrange cell kernel's columns (instance, chunk, segment); not schema-csts
+  bool columns;                 // the Lagrange cell kernel takes columns (FP64 without schema-csts, layers that fill them)
+  const int4* cwork;            // and their work table (instance, chunk, segment)
   int ncwork;
   int col_strip;                // the longest strip of nodes its instances need
   const int4* fwork;            // schema-csts: face work table (instance, chunk of 128 faces of all directions)
@@ -269,6 +270,13 @@ __global__ void k_dt_finish_ext(Scalars* S, Phys ph, const unsigned long long* m
 constexpr int kColThreads = 128;
 constexpr int kColLayers = 8;
 __host__ __device__ __forceinline__ int col_blocks(int nx, int ny) { return (nx * ny + kColThreads - 1) / kColThreads; }
+// Columns pay where the layers fill the threads of their blocks: `threads` is
+// kColThreads x col_blocks x nz, over one mesh or a batch.  Measured on B200, a cycle
+// of FP64, columns against one thread a cell: 2x2x20000 (3 % filled) 510 -> 328 us,
+// 5x5x4000 (20 %) 166 -> 139, 12x12x800 (56 %) 122 -> 113, 20x20x300 (78 %) 108 ->
+// 106, 18x18x400 (84 %) 117 -> 116, 23x23x300 (83 %) 122 -> 123, 22x22x300 (95 %) 113
+// -> 120, 30x30x200 (88 %) 144 -> 151.
+__host__ __device__ __forceinline__ bool col_filled(long long cells, long long threads) { return 5 * cells >= 4 * threads; }
 __host__ __device__ __forceinline__ int col_segments(int nx, int ny, int nz) {
   const int by_len = (nz + kColLayers - 1) / kColLayers, fill = (444 + col_blocks(nx, ny) - 1) / col_blocks(nx, ny);
   const int want = fill < nz ? fill : nz;

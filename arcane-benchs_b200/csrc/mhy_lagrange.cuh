@@ -711,8 +711,13 @@ __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat
 
 // Whether a context's FP64 cell kernel takes columns: not on small meshes, whose
 // few blocks do not hide the copy of the first planes (100x5x5: 13.9 us against
-// 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1).
+// 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1), and not
+// where the layers leave threads idle (col_filled).
 constexpr long long kColMinCells = 65536;
+inline bool takes_columns(const CycleArgs& a) {
+  return !a.ph.precision && a.dm.C >= kColMinCells &&
+         col_filled(a.dm.C, (long long)kColThreads * col_blocks(a.dm.nx, a.dm.ny) * a.dm.nz);
+}
 
 template <int K, bool HC, bool NEWTON>
 static void launch_columns(const CycleArgs& a, cudaStream_t s) {
@@ -729,7 +734,7 @@ static void launch_columns(const CycleArgs& a, cudaStream_t s) {
 template <int K, bool NEWTON>
 static void launch_cells(const CycleArgs& a, cudaStream_t s) {
   const bool hc = a.fd.h != nullptr;               // cell widths: order 3 or the generalised limiters
-  if (!a.ph.precision && a.dm.C >= kColMinCells) {
+  if (takes_columns(a)) {
     if (hc) launch_columns<K, true, NEWTON>(a, s);
     else launch_columns<K, false, NEWTON>(a, s);
     return;
@@ -758,13 +763,7 @@ static void launch_bat_columns(const BatchPlan& P, cudaStream_t s, KernelMarks* 
         P.descs, P.cwork, P.ncwork);
   mark(m, BK_LCELLS, s);
 }
-template <int K, bool HC>
-static void launch_bat_columns(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
-  if (P.newton) launch_bat_columns<K, HC, true>(P, s, m);
-  else launch_bat_columns<K, HC, false>(P, s, m);
-}
-
-// A batch's mixed form and schema-csts: the cell tiles of BK_LCELLS.
+// What of a batch takes no columns: the cell tiles of BK_LCELLS.
 template <int K, typename R, bool HC, bool CSTS, bool NEWTON>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_lagrange_cells(const CycleArgs* __restrict__ D,
                                                                                    const int4* __restrict__ W, int nw) {
@@ -775,6 +774,29 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) k_bat_lagrange_ce
                                               a.st.cs, a.st.mass, a.cqs, CSTS ? nullptr : a.cqs32, a.L, a.U[0], a.xc,
                                               a.fd, a.env, a.Vlag, t.y, t.z, t.w, a.vnb, a.pf);
   }
+}
+
+template <int K, typename R, bool HC, bool CSTS, bool NEWTON>
+static void launch_bat_tiles(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  auto kern = k_bat_lagrange_cells<K, R, HC, CSTS, NEWTON>;
+  if (P.nwork[BK_LCELLS] > 0)
+    kern<<<persistent_grid((const void*)kern, 128, 0, P.nwork[BK_LCELLS], P.occ_pct[BK_LCELLS]), 128, 0, s>>>(
+        P.descs, P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+  mark(m, BK_LCELLS, s);
+}
+
+// The cell kernel of a batch, all but schema-csts.
+template <int K, typename R, bool HC, bool NEWTON>
+static void launch_bat_cells(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  if constexpr (sizeof(R) == 8) {
+    if (P.columns) { launch_bat_columns<K, HC, NEWTON>(P, s, m); return; }
+  }
+  launch_bat_tiles<K, R, HC, false, NEWTON>(P, s, m);
+}
+template <int K, typename R, bool HC>
+static void launch_bat_cells(const BatchPlan& P, cudaStream_t s, KernelMarks* m) {
+  if (P.newton) launch_bat_cells<K, R, HC, true>(P, s, m);
+  else launch_bat_cells<K, R, HC, false>(P, s, m);
 }
 
 }  // namespace mhy

@@ -1245,18 +1245,12 @@ static void batch_cycle_env(const BatchPlan& P, int sens, cudaStream_t s, Kernel
   bool done = false;
   if constexpr (sizeof(R) == 8) {
     if (P.csts) {   // schema-csts: the cell kernel's CSTS form, then the forward step and the face velocities
-      bat_env_launch(k_bat_lagrange_cells<K, double, HC, true, false>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
-                     P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
+      launch_bat_tiles<K, double, HC, true, false>(P, s, m);
       launch_bat_csts_forward(P, s);
       done = true;
     }
   }
-  if (!done) {
-    if constexpr (sizeof(R) == 8) launch_bat_columns<K, HC>(P, s, m);
-    else bat_env_launch(P.newton ? k_bat_lagrange_cells<K, float, false, false, true>
-                                 : k_bat_lagrange_cells<K, float, false, false, false>, 128, 0, P, BK_LCELLS, BK_LCELLS, s, m, P.descs,
-                        P.work[BK_LCELLS], P.nwork[BK_LCELLS]);
-  }
+  if (!done) launch_bat_cells<K, R, sizeof(R) == 8 && HC>(P, s, m);
   int prev = 0;
   for (int it = 0; it < 3; ++it) {
     const int d = (it + sens) % 3;
