@@ -724,7 +724,7 @@ struct mhy_batch {
   CycleArgs* d_descs = nullptr;
   int4* d_work[BK_COUNT] = {};
   int4* d_mwork[BK_COUNT] = {};                 // marching sweeps
-  int4* d_cwork = nullptr;                      // the Lagrange cell kernel's columns
+  int4* d_cwork = nullptr;                      // the Lagrange cell kernel's columns (BatchPlan::columns)
   int4* d_o3work[3] = {};                       // order 3: face work tables per direction
   int4* d_fwork = nullptr;                      // schema-csts: face work table (all directions)
   int col_order = 0;                            // and of the columns
@@ -851,22 +851,22 @@ int mhy_batch_create(int n, const mhy_mesh_desc* meshes, const mhy_options* opts
     b->plan.mwork[k] = b->d_mwork[k];
     b->plan.nmwork[k] = (int)mw.size();
   }
-  {
+  long long cells = 0, threads = 0;
+  for (const mhy_ctx* c : b->inst) {
+    int blocks, segments, strip;
+    batch_column_shape(c->dm, blocks, segments, strip);
+    b->plan.col_strip = std::max(b->plan.col_strip, strip);
+    cells += c->dm.C;
+    threads += (long long)kColThreads * blocks * c->dm.nz;
+  }
+  b->plan.columns = opts[0].precision == 0 && !opts[0].schema_csts && col_filled(cells, threads);
+  if (b->plan.columns) {
     const std::vector<int4> w = build_work(b->inst, kColumns, 0, kLineWarps, false);
     err = cudaMalloc(&b->d_cwork, w.size() * sizeof(int4));
     if (err == cudaSuccess) err = cudaMemcpy(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
     b->plan.cwork = b->d_cwork;
     b->plan.ncwork = (int)w.size();
-    long long cells = 0, threads = 0;
-    for (const mhy_ctx* c : b->inst) {
-      int blocks, segments, strip;
-      batch_column_shape(c->dm, blocks, segments, strip);
-      b->plan.col_strip = std::max(b->plan.col_strip, strip);
-      cells += c->dm.C;
-      threads += (long long)kColThreads * blocks * c->dm.nz;
-    }
-    b->plan.columns = opts[0].precision == 0 && !opts[0].schema_csts && col_filled(cells, threads);
   }
   err = cudaMalloc(&b->d_descs, n * sizeof(CycleArgs));
   if (err != cudaSuccess) { mhy_batch_destroy(b); return fail(MHY_ERR_OOM, cudaGetErrorString(err)); }
@@ -1070,7 +1070,7 @@ int apply_tuning(mhy_batch* b, const mhy_tuning& t) {
     b->plan.lines[k] = t.lines_per_block[k];
     b->plan.nwork[k] = (int)w.size();
   }
-  if (t.order[BK_LCELLS] != b->col_order) {
+  if (b->plan.columns && t.order[BK_LCELLS] != b->col_order) {
     const std::vector<int4> w = build_work(b->inst, kColumns, t.order[BK_LCELLS], kLineWarps, false);
     MHY_CUDA(cudaMemcpyAsync(b->d_cwork, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
     MHY_CUDA(cudaStreamSynchronize(b->stream));
