@@ -114,9 +114,9 @@ __device__ __forceinline__ void corner_vectors(const Vec3<T> x[8], Finish&& fini
 }
 
 // Remap face data from a cell's nodes (PrepareRemap.cc:41-55, 105-117;
-// RemapADIService.cc:710): for the low face of each direction |A| along d, u_f and (x_f - x_c).n0 with this cell as the next cell;
-// for the high face (x_f - x_c).n0 with this cell as the
-// previous one.  Face node order: X (0,3,7,4), Y (0,1,5,4), Z (0,1,2,3) low;
+// RemapADIService.cc:710): for the low face of each direction |A| along d, u_f and
+// (x_f - x_c).n0 with this cell as the next cell; for the high face (x_f - x_c).n0
+// with this cell as the previous one.  Face node order: X (0,3,7,4), Y (0,1,5,4), Z (0,1,2,3) low;
 // X (1,2,6,5), Y (3,2,6,7), Z (4,5,6,7) high, in SN_trigo cell-node numbers.
 // In FP64 the values of boundary faces are written too and read by nobody:
 // without a branch the faces' arithmetic overlaps the chain of the thermodynamics.
@@ -545,7 +545,7 @@ constexpr int kColPriv = 24;         // doubles a cell: 18 normals (low and high
 // the block's first cell onwards and from one row up; a strip holds the block's
 // cells, one node more a row that it touches and one for its last cell.  Two
 // lengths, known at compile time so that a cell's nodes lie at fixed offsets:
-// one for rows of 26 cells and more, one for any row of two cells and more.
+// one for rows of 22 cells and more, one for any row of two cells and more.
 constexpr int kColStrip = 136, kColStripWide = 200;
 __host__ __device__ __forceinline__ int col_strip(int nx) {
   return kColThreads + (kColThreads + nx - 2) / nx + 2 <= kColStrip ? kColStrip : kColStripWide;
@@ -712,7 +712,8 @@ __global__ void __launch_bounds__(kColThreads, STRIP == kColStrip ? 3 : 2) k_bat
 // Whether a context's FP64 cell kernel takes columns: not on small meshes, whose
 // few blocks do not hide the copy of the first planes (100x5x5: 13.9 us against
 // 9.9 us for one thread a cell; 37^3, 50,653 cells: 14.8 against 13.1), and not
-// where the layers leave threads idle (col_filled).
+// where the layers leave threads idle (col_filled).  The mixed form keeps one
+// thread a cell: in columns it took 236 to 294 us on Sedov 128^3 against 219 to 230.
 constexpr long long kColMinCells = 65536;
 inline bool takes_columns(const CycleArgs& a) {
   return !a.ph.precision && a.dm.C >= kColMinCells &&

@@ -23,7 +23,8 @@ __host__ __device__ __forceinline__ void march_range(int n, int seg, int nseg, i
 
 // Segments of a line of n items over a plane of `points` lines: `len` items
 // a segment, shorter where that many threads would not fill the chip
-// (kMarchFill threads), but not below 4 items.
+// (kMarchFill threads), down to (n + 3) / 4 segments: 4 or 3 items each (2 and 3
+// on a line of 5).
 constexpr int kMarchFill = 148 * 4 * kMarchThreads;
 __host__ __device__ __forceinline__ int march_segments(int n, int points, int len) {
   const int by_len = (n + len - 1) / len, fill = (kMarchFill + points - 1) / points, most = (n + 3) / 4;

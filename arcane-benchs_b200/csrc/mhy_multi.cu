@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(32 * W, kEnvMinBlocks * kLineWarps / W) k_env_
 // (RemapADIService.cc:583-641, Remap-ordre-3.cc:7-131), one thread per face.
 // Phi of the six cells around an inner face (clamped at the ends of the
 // line) as the sweeps form it (U over the Lagrangian volume on the first
-// sweep, over the sum of the environment volumes afterwards), o3_flux per
+// sweep, over the sum of the environment volumes afterwards), o3_value per
 // component; then, unless the two cells are pure cells of one environment,
 // each environment's density and energy face values are rescaled by the
 // upwind cell's ratios (R:623-641).  A cell is mixed when more than one
