@@ -6,6 +6,7 @@ operation rounds exactly as written (the CPU oracle is built with
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import pathlib
 import shutil
@@ -42,17 +43,23 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
     if not force and not _stale():
         return LIB
     LIB_DIR.mkdir(exist_ok=True)
-    objs = []
-    logs = []
-    for src in SOURCES:
+
+    def compile_one(src):
         obj = LIB_DIR / (pathlib.Path(src).stem + ".o")
         cmd = [nvcc(), *ARCH, *FLAGS, "-rdc=false", "-c", str(CSRC / src), "-o", str(obj)]
-        r = subprocess.run(cmd, capture_output=True, text=True)
+        return str(obj), subprocess.run(cmd, capture_output=True, text=True)
+
+    objs = []
+    logs = []
+    # side by side: two of the files take most of the time
+    with concurrent.futures.ThreadPoolExecutor(len(SOURCES)) as pool:
+        done = list(pool.map(compile_one, SOURCES))
+    for src, (obj, r) in zip(SOURCES, done):
         logs.append(r.stdout + r.stderr)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError(f"nvcc failed on {src}")
-        objs.append(str(obj))
+        objs.append(obj)
     cmd = [nvcc(), *ARCH, "-shared", "-o", str(LIB), *objs, "-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
